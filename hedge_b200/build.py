@@ -15,6 +15,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhedge_b200.so")
 SOURCES = ["api.cu", "rhs_simt.cu", "rhs_split.cu", "norm.cu", "adjoint.cu", "ensemble.cu",
            "waitcheck.cu", "rhs_quad.cu"]
+# the FP64 tensor-core kernel's instances, in parts that compile side by side
+FP64_PARTS = 5
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -41,11 +43,14 @@ def build(force=False, verbose=False, extra_flags=()):
     build_dir = os.path.join(HERE, "_build")
     os.makedirs(build_dir, exist_ok=True)
     procs = []
-    for src in SOURCES:
-        obj = os.path.join(build_dir, src.replace(".cu", ".o"))
+    units = [(src, src.replace(".cu", ".o"), []) for src in SOURCES]
+    units += [("rhs_fp64.cu", "rhs_fp64_%d.o" % p, ["-DHB_FP64_PART=%d" % p])
+              for p in range(FP64_PARTS)]
+    for src, obj, defines in units:
+        obj = os.path.join(build_dir, obj)
         cmd = [nvcc(), "-std=c++17", "-O3", *ARCH, "-lineinfo", "-Xcompiler", "-fPIC",
                "-Xptxas", "-v" if verbose else "-O3", "--expt-relaxed-constexpr",
-               *extra_flags, "-c", os.path.join(CSRC, src), "-o", obj]
+               *extra_flags, *defines, "-c", os.path.join(CSRC, src), "-o", obj]
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE,
                                             stderr=subprocess.STDOUT)))
         objs.append(obj)

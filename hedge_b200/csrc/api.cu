@@ -291,7 +291,7 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
   hb_status st;
   auto bail = [&](hb_status s) {
     cudaFree(op->conn); cudaFree(op->err_flag);
-    cudaFree(op->quad64); cudaFree(op->elmax);
+    cudaFree(op->quad64); cudaFree(op->elmax); cudaFree(op->afrag);
     free_split(op);
     delete op;
     return s;
@@ -318,7 +318,8 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
       st = prepare_simt(op);
     }
   } else {
-    st = prepare_simt(op);
+    st = op->precision == HB_PREC_FP64 ? prepare_f64(op) : HB_ERR_UNSUPPORTED;
+    if (st == HB_ERR_UNSUPPORTED) st = prepare_simt(op);
   }
   if (st) return bail(st);
   *out = reinterpret_cast<hb_op*>(op);
@@ -331,7 +332,7 @@ hb_status hb_op_destroy(hb_op* handle) {
   DeviceGuard g(op->d->device);
   cudaFree(op->conn);
   cudaFree(op->err_flag);
-  cudaFree(op->quad64); cudaFree(op->elmax);
+  cudaFree(op->quad64); cudaFree(op->elmax); cudaFree(op->afrag);
   free_split(op);
   delete op;
   return HB_OK;
@@ -373,6 +374,8 @@ static hb_status run(Op* op, int mode, double a, double b, double dt, const void
   }
   if (op->split)
     return launch_split(op, mode, a, b, dt, q_in, q_out, res, coeff, bdry, source, e0, e1, s);
+  if (op->afrag)
+    return launch_f64(op, mode, a, b, dt, q_in, q_out, res, coeff, bdry, source, e0, e1, s);
   return launch_simt(op, mode, a, b, dt, q_in, q_out, res, coeff, bdry, source, e0, e1, s);
 }
 

@@ -95,6 +95,9 @@ struct Op {
   int grid = 0;
   int ops_in_smem = 1;
   int blocks_per_sm = 0;
+  // FP64 operators of order 1 to 7: [D | LIFT] as FP64 matrix fragments
+  double* afrag = nullptr;
+  int f64_slots[2] = {0, 0};   // CTAs resident on the GPU: fixed, variable material
   // split-precision operator planes (BF16X3)
   void* split_ops = nullptr;
   // quadrature operator (variable-coefficient advection): point counts, the
@@ -130,6 +133,13 @@ hb_status launch_simt(Op* op, int mode, double a, double b, double dt,
                       const double* coeff, const double* bdry,
                       const double* source, int64_t e0, int64_t e1, cudaStream_t s);
 hb_status prepare_simt(Op* op);
+
+// FP64 tensor-core kernel (rhs_fp64.cu): operators of order 1 to 7; prepare
+// refuses the others (HB_ERR_UNSUPPORTED), which run on the CUDA cores
+hb_status launch_f64(Op* op, int mode, double ra, double rb, double dt, const void* q_in,
+                     void* q_out, void* res, const double* coeff, const double* bdry,
+                     const double* source, int64_t e0, int64_t e1, cudaStream_t s);
+hb_status prepare_f64(Op* op);
 
 // quadrature kernel (rhs_quad.cu); vel = the velocity field [dim][K*Np]
 hb_status prepare_quad(Op* op);
