@@ -65,7 +65,7 @@ EXPORTED = [
     "hb_rhs", "hb_lsrk_stage", "hb_rhs_elements", "hb_lsrk_stage_elements", "hb_lincomb",
     "hb_gather_map", "hb_op_check",
     "hb_op_launch_info", "hb_norm", "hb_norm_noalloc", "hb_rhs_adjoint_work_size",
-    "hb_rhs_adjoint", "hb_batch_create", "hb_batch_destroy", "hb_batch_stage",
+    "hb_rhs_adjoint", "hb_adjoint_stage", "hb_batch_create", "hb_batch_destroy", "hb_batch_stage",
     "hb_batch_info", "hb_batch_check", "hb_op_set_halo", "hb_pack",
     "hb_op_wait_selftest", "hb_last_error_string",
 ]
@@ -103,6 +103,7 @@ def load(path=LIB_PATH):
             "hb_norm_noalloc": [i64, i32, i32, i32, vp, vp, vp, vp, vp],
             "hb_rhs_adjoint_work_size": [vp, vp],
             "hb_rhs_adjoint": [vp, vp, vp, vp, vp, vp, vp, vp],
+            "hb_adjoint_stage": [vp, d, d, d, vp, vp, vp, vp, vp, vp, vp],
             "hb_batch_create": [vp, i32, vp],
             "hb_batch_destroy": [vp],
             "hb_batch_stage": [vp, d, d, i32, vp],

@@ -199,13 +199,8 @@ class ReceiverTraces:
                             keep = stages[n - s0]
                             lres = torch.zeros_like(lq)
                             for s in range(4, -1, -1):
-                                lres = lres + RK4B[s] * lq
-                                q_bar, cb = comp.adjoint(lres, q=keep[s], coeff=cc,
-                                                         want_c=want_c)
-                                lq = lq + dt * q_bar
-                                if want_c:
-                                    c_bar = c_bar + dt * cb
-                                lres = RK4A[s] * lres
+                                comp.adjoint_stage(RK4A[s], RK4B[s], dt, lres, lq,
+                                                   q=keep[s], coeff=cc, c_bar=c_bar)
                             lq = lq + rec.transpose(g[n], lq)
                     q0_bar = lq.reshape(ctx.checkpoints[0].shape)
                     return q0_bar, c_bar, None, None, None, None, None, None

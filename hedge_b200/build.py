@@ -15,8 +15,9 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhedge_b200.so")
 SOURCES = ["api.cu", "rhs_simt.cu", "rhs_split.cu", "norm.cu", "adjoint.cu", "ensemble.cu",
            "waitcheck.cu", "rhs_quad.cu"]
-# the FP64 tensor-core kernel's instances, in parts that compile side by side
-FP64_PARTS = 5
+# the FP64 tensor-core kernels' instances, in parts that compile side by side:
+# (source, macro that selects the part, parts)
+PARTS = [("rhs_fp64.cu", "HB_FP64_PART", 5), ("adjoint_fp64.cu", "HB_ADJ_PART", 4)]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -44,8 +45,8 @@ def build(force=False, verbose=False, extra_flags=()):
     os.makedirs(build_dir, exist_ok=True)
     procs = []
     units = [(src, src.replace(".cu", ".o"), []) for src in SOURCES]
-    units += [("rhs_fp64.cu", "rhs_fp64_%d.o" % p, ["-DHB_FP64_PART=%d" % p])
-              for p in range(FP64_PARTS)]
+    units += [(src, src.replace(".cu", "_%d.o" % p), ["-D%s=%d" % (macro, p)])
+              for src, macro, n in PARTS for p in range(n)]
     for src, obj, defines in units:
         obj = os.path.join(build_dir, obj)
         cmd = [nvcc(), "-std=c++17", "-O3", *ARCH, "-lineinfo", "-Xcompiler", "-fPIC",

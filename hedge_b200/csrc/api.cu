@@ -291,7 +291,7 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
   hb_status st;
   auto bail = [&](hb_status s) {
     cudaFree(op->conn); cudaFree(op->err_flag);
-    cudaFree(op->quad64); cudaFree(op->elmax); cudaFree(op->afrag);
+    cudaFree(op->quad64); cudaFree(op->elmax); cudaFree(op->afrag); cudaFree(op->adjfrag);
     free_split(op);
     delete op;
     return s;
@@ -321,6 +321,10 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
     st = op->precision == HB_PREC_FP64 ? prepare_f64(op) : HB_ERR_UNSUPPORTED;
     if (st == HB_ERR_UNSUPPORTED) st = prepare_simt(op);
   }
+  if (!st && model != HB_MODEL_VARADV && d->order <= 7) {
+    st = prepare_adjoint_f64(op);
+    if (st == HB_ERR_UNSUPPORTED) st = HB_OK;   // the CUDA-core adjoint
+  }
   if (st) return bail(st);
   *out = reinterpret_cast<hb_op*>(op);
   return HB_OK;
@@ -332,7 +336,7 @@ hb_status hb_op_destroy(hb_op* handle) {
   DeviceGuard g(op->d->device);
   cudaFree(op->conn);
   cudaFree(op->err_flag);
-  cudaFree(op->quad64); cudaFree(op->elmax); cudaFree(op->afrag);
+  cudaFree(op->quad64); cudaFree(op->elmax); cudaFree(op->afrag); cudaFree(op->adjfrag);
   free_split(op);
   delete op;
   return HB_OK;
@@ -471,12 +475,8 @@ hb_status hb_rhs_adjoint_work_size(hb_op* handle, int64_t* bytes) {
   return HB_OK;
 }
 
-hb_status hb_rhs_adjoint(hb_op* handle, const double* q, const double* lam, double* q_bar,
-                         double* c_bar, const double* coeff, void* work, void* stream) {
-  if (!handle) return fail(HB_ERR_INVALID_ARGUMENT, "null operator");
-  Op* op = reinterpret_cast<Op*>(handle);
-  if (!lam || !q_bar || !work) return fail(HB_ERR_INVALID_ARGUMENT, "null argument");
-  if (lam == q_bar) return fail(HB_ERR_INVALID_ARGUMENT, "q_bar aliases lam");
+static hb_status check_adjoint(Op* op, const double* q, const double* c_bar,
+                               const double* coeff) {
   if (op->model == HB_MODEL_VARWAVE && !coeff)
     return fail(HB_ERR_INVALID_ARGUMENT, "variable-velocity wave needs the c field");
   if (c_bar && op->model != HB_MODEL_VARWAVE)
@@ -485,10 +485,40 @@ hb_status hb_rhs_adjoint(hb_op* handle, const double* q, const double* lam, doub
                 op->model == HB_MODEL_MAXWELL_TE))
     return fail(HB_ERR_UNSUPPORTED, "adjoint: Maxwell with variable material is not built");
   if (c_bar && !q) return fail(HB_ERR_INVALID_ARGUMENT, "c_bar needs the state q");
+  return HB_OK;
+}
+
+hb_status hb_rhs_adjoint(hb_op* handle, const double* q, const double* lam, double* q_bar,
+                         double* c_bar, const double* coeff, void* work, void* stream) {
+  if (!handle) return fail(HB_ERR_INVALID_ARGUMENT, "null operator");
+  Op* op = reinterpret_cast<Op*>(handle);
+  if (!lam || !q_bar || !work) return fail(HB_ERR_INVALID_ARGUMENT, "null argument");
+  if (lam == q_bar) return fail(HB_ERR_INVALID_ARGUMENT, "q_bar aliases lam");
+  const hb_status st = check_adjoint(op, q, c_bar, coeff);
+  if (st) return st;
   DeviceGuard g(op->d->device);
   if (!g.ok) return fail(HB_ERR_CUDA, "cannot select the CUDA device");
   return launch_adjoint(op, q, lam, q_bar, c_bar, coeff, static_cast<double*>(work),
                         reinterpret_cast<cudaStream_t>(stream));
+}
+
+hb_status hb_adjoint_stage(hb_op* handle, double a, double b, double dt, const double* q,
+                           double* lam, double* lq, double* c_bar, const double* coeff,
+                           void* work, void* stream) {
+  if (!handle) return fail(HB_ERR_INVALID_ARGUMENT, "null operator");
+  Op* op = reinterpret_cast<Op*>(handle);
+  if (!lam || !lq || !work) return fail(HB_ERR_INVALID_ARGUMENT, "null argument");
+  if (lam == lq || q == lam || q == lq)
+    return fail(HB_ERR_INVALID_ARGUMENT, "adjoint stage: aliasing vectors");
+  const hb_status st = check_adjoint(op, q, c_bar, coeff);
+  if (st) return st;
+  if (!op->adjfrag)
+    return fail(HB_ERR_UNSUPPORTED, "adjoint stage: orders 1 to 7 (compose it from "
+                                    "hb_rhs_adjoint)");
+  DeviceGuard g(op->d->device);
+  if (!g.ok) return fail(HB_ERR_CUDA, "cannot select the CUDA device");
+  return launch_adjoint_stage(op, a, b, dt, q, lam, lq, c_bar, coeff, static_cast<double*>(work),
+                              reinterpret_cast<cudaStream_t>(stream));
 }
 
 hb_status hb_op_set_halo(hb_op* handle, const void* halo, const double* halo_coeff) {

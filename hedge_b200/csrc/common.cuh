@@ -98,6 +98,10 @@ struct Op {
   // FP64 operators of order 1 to 7: [D | LIFT] as FP64 matrix fragments
   double* afrag = nullptr;
   int f64_slots[2] = {0, 0};   // CTAs resident on the GPU: fixed, variable material
+  // the adjoint of an operator of order 1 to 7: fragments and resident CTAs
+  // (lift pass, element pass without and with the c gradient)
+  double* adjfrag = nullptr;
+  int adj_slots[3] = {0, 0, 0};
   // split-precision operator planes (BF16X3)
   void* split_ops = nullptr;
   // quadrature operator (variable-coefficient advection): point counts, the
@@ -121,6 +125,15 @@ hb_status launch_norm(int64_t K, int np, int nfields, int dtype, const double* m
 int64_t adjoint_work_bytes(const Op* op);
 hb_status launch_adjoint(Op* op, const double* q, const double* lam, double* q_bar,
                          double* c_bar, const double* coeff, double* work, cudaStream_t s);
+
+// the same on the FP64 tensor cores (adjoint_fp64.cu), operators of order 1 to
+// 7, and one stage of the reversed LSRK recurrences around it, in place
+hb_status prepare_adjoint_f64(Op* op);
+hb_status launch_adjoint_f64(Op* op, const double* q, const double* lam, double* q_bar,
+                             double* c_bar, const double* coeff, double* work, cudaStream_t s);
+hb_status launch_adjoint_stage(Op* op, double ra, double rb, double dt, const double* q,
+                               double* lam, double* lq, double* c_bar, const double* coeff,
+                               double* work, cudaStream_t s);
 
 // gather for halo exchange (rhs_simt.cu): dst[j][f] = src[f][idx[j]]
 hb_status launch_pack(int64_t n, int dtype, int nfields, int64_t field_stride,

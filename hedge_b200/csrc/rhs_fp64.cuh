@@ -77,6 +77,10 @@ struct F64Shape {
   // few node tiles leave registers for more column tiles (and the batch then
   // has a node or a face point for every thread)
   static constexpr int RN = MT == 1 ? 8 : MT == 2 ? 4 : 2;
+  // two steps in flight where the tile and the model leave registers (stage
+  // times: 2D wave N = 3, K = 684 4.6 -> 4.3 us; Maxwell N = 2, K = 48000 58.6 ->
+  // 61.4 us, so not there)
+  static constexpr int UNROLL = MT <= 3 && F <= 3 ? 2 : 1;
   static constexpr int NGW = 2;
   // from 11 node tiles a CTA fills the SM: four k shares give it 8 warps
   static constexpr int KG = MT >= 11 ? 4 : 2;
@@ -131,19 +135,6 @@ struct F64Args {
   int mode;                  // 0: write rhs, 1: LSRK stage
   ModelParams mp;
 };
-
-__device__ __forceinline__ void cp_async8(void* smem, const void* g) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
-                   (uint32_t)__cvta_generic_to_shared(smem)),
-               "l"(g)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
 
 // VM: Maxwell with variable material (coeff = [eps | mu])
 template <int MODEL, int DIM, int ORDER, bool VM>
@@ -313,30 +304,15 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
               }
         }
       };
-      // a node tile's operator fragment for the next step is requested as
-      // soon as its last product of this step is issued
-      double2 af[MT];
-#pragma unroll
-      for (int m = 0; m < MT; ++m) af[m] = __ldg(ap + m * 32);
-      for (int s = s0; s < s1; ++s) {
-        if (C != 0 && s == S::KVP / 8) scale_c();
-        double2 b[RN];
-#pragma unroll
-        for (int c = 0; c < RN; ++c) b[c] = *reinterpret_cast<const double2*>(zp + c * 8 * LDZ);
-        ap += s + 1 < s1 ? MT * 32 : 0;   // the last step reloads its own
-        zp += 8;
-#pragma unroll
-        for (int m = 0; m < MT; ++m)
-#pragma unroll
-          for (int c = 0; c < RN; ++c) dmma(acc[m][c], af[m].x, b[c].x);
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-#pragma unroll
-          for (int c = 0; c < RN; ++c) dmma(acc[m][c], af[m].y, b[c].y);
-          af[m] = __ldg(ap + m * 32);
-        }
+      if constexpr (C != 0) {
+        constexpr int SV = S::KVP / 8;
+        const int nv = s1 < SV ? s1 - s0 : s0 < SV ? SV - s0 : 0;   // volume steps
+        dmma_steps<MT, RN, LDZ, S::UNROLL>(acc, ap, zp, nv);
+        if (nv > 0) scale_c();
+        dmma_steps<MT, RN, LDZ, S::UNROLL>(acc, ap + (size_t)nv * MT * 32, zp + 8 * nv, s1 - s0 - nv);
+      } else {
+        dmma_steps<MT, RN, LDZ, S::UNROLL>(acc, ap, zp, s1 - s0);
       }
-      if (C != 0 && s1 <= S::KVP / 8) scale_c();
     }
     __syncthreads();   // all warps are done reading Z
     if (work) {
@@ -424,16 +400,6 @@ struct F64Call {
   bool configure;
 };
 
-// Elements per batch of a launch over n elements: EB, evened out over whole
-// rounds of the grid; on a mesh smaller than one round fewer, down to one tile
-// of 8 columns, so that every SM has work (684 triangles of N = 3: 228 CTAs
-// and 4.2 us a stage, where batches of 25 made 28 CTAs and 8.3 us)
-inline int f64_batch(int64_t n, int eb, int fields, int64_t slots) {
-  const int64_t rounds = (n + eb * slots - 1) / (eb * slots);
-  const int64_t even = (n + rounds * slots - 1) / (rounds * slots);
-  return (int)std::min<int64_t>(eb, std::max<int64_t>(even, (8 + fields - 1) / fields));
-}
-
 template <int MODEL, int DIM, int ORDER, bool VM>
 hb_status f64_one(const F64Call& c) {
   using S = F64Shape<MODEL, DIM, ORDER>;
@@ -455,7 +421,7 @@ hb_status f64_one(const F64Call& c) {
     if (per_sm < 1) return fail(HB_ERR_UNSUPPORTED, "FP64 kernel does not fit on an SM");
     op->f64_slots[VM] = sms * per_sm;
     if constexpr (VM) return HB_OK;   // the rest is the fixed-material kernel's
-    op->elems_per_block = f64_batch(d->K, S::EB, S::F, op->f64_slots[0]);
+    op->elems_per_block = dmma_batch(d->K, S::EB, S::F, op->f64_slots[0]);
     op->blocks_per_sm = per_sm;
     op->threads = S::THREADS;
     op->smem = S::total;
@@ -473,8 +439,7 @@ hb_status f64_one(const F64Call& c) {
                               ? lift + (size_t)(k - S::KVP) * S::NP : nullptr;
       if (!row) continue;
       for (int i = 0; i < S::NP; ++i)
-        fr[(((size_t)(k / 8) * S::MT + i / 8) * 32 + (i % 8) * 4 + (k % 8) / 2) * 2 + (k & 1)] =
-            row[i];
+        fr[dmma_afrag(i, k, S::MT)] = row[i];
     }
     if (cudaMalloc(&op->afrag, sizeof(double) * fr.size()) != cudaSuccess ||
         cudaMemcpy(op->afrag, fr.data(), sizeof(double) * fr.size(), cudaMemcpyHostToDevice) !=
@@ -487,7 +452,7 @@ hb_status f64_one(const F64Call& c) {
   a.e_begin = c.e0;
   a.e_end = c.e1;
   const int slots = op->f64_slots[VM];
-  a.E = f64_batch(c.e1 - c.e0, S::EB, S::F, slots);
+  a.E = dmma_batch(c.e1 - c.e0, S::EB, S::F, slots);
   a.nbatch = (c.e1 - c.e0 + a.E - 1) / a.E;
   a.nperm = d->nperm;
   a.face.K = d->K;

@@ -710,18 +710,50 @@ class CompiledOperator:
             raise ValueError("c gradient: variable-velocity wave, with the state q")
         q_bar = torch.empty_like(lam)
         c_bar = torch.empty(len(d), dtype=torch.float64, device=d.device) if want_c else None
-        nbytes = C.c_int64()
-        _native.check(self._lib.hb_rhs_adjoint_work_size(self._handle, C.byref(nbytes)))
-        work = getattr(self, "_adj_work", None)
-        if work is None or work.numel() * 8 < nbytes.value:
-            work = torch.empty((nbytes.value + 7) // 8, dtype=torch.float64, device=d.device)
-            self._adj_work = work
+        work = self._adjoint_work()
         c = self._coeff if coeff is None else coeff
         _native.check(self._lib.hb_rhs_adjoint(
             self._handle, q.data_ptr() if q is not None else None, lam.data_ptr(),
             q_bar.data_ptr(), c_bar.data_ptr() if c_bar is not None else None,
             c.data_ptr() if c is not None else None, work.data_ptr(), self._stream()))
         return q_bar, c_bar
+
+    def _adjoint_work(self):
+        torch = _torch()
+        nbytes = C.c_int64()
+        _native.check(self._lib.hb_rhs_adjoint_work_size(self._handle, C.byref(nbytes)))
+        work = getattr(self, "_adj_work", None)
+        if work is None or work.numel() * 8 < nbytes.value:
+            work = torch.empty((nbytes.value + 7) // 8, dtype=torch.float64,
+                               device=self.discr.device)
+            self._adj_work = work
+        return work
+
+    def adjoint_stage(self, a, b, dt, lam, lq, q=None, coeff=None, c_bar=None):
+        """One stage of the reversed LSRK recurrences, in place on the
+        contiguous FP64 device tensors lam, lq [F, K*Np] and, unless None,
+        c_bar [K*Np]:
+
+            lam += b lq;  lq += dt (dR/dq)^T lam;  c_bar += dt (dR/dc)^T lam;
+            lam *= a
+
+        (hb_adjoint_stage: two launches; beyond order 7 composed from
+        ``adjoint``)."""
+        if self.discr.order > 7:
+            lam.add_(lq, alpha=b)
+            q_bar, cb = self.adjoint(lam, q=q, coeff=coeff, want_c=c_bar is not None)
+            lq.add_(q_bar, alpha=dt)
+            if c_bar is not None:
+                c_bar.add_(cb, alpha=dt)
+            lam.mul_(a)
+            return
+        c = self._coeff if coeff is None else coeff
+        _native.check(self._lib.hb_adjoint_stage(
+            self._handle, float(a), float(b), float(dt),
+            q.data_ptr() if q is not None else None, lam.data_ptr(), lq.data_ptr(),
+            c_bar.data_ptr() if c_bar is not None else None,
+            c.data_ptr() if c is not None else None, self._adjoint_work().data_ptr(),
+            self._stream()))
 
     def check(self):
         """Synchronise and raise if a kernel flagged bad input."""

@@ -250,6 +250,17 @@ hb_status hb_rhs_adjoint_work_size(hb_op* op, int64_t* bytes);
 hb_status hb_rhs_adjoint(hb_op* op, const double* q, const double* lam, double* q_bar,
                          double* c_bar, const double* coeff, void* work, void* stream);
 
+/* One stage of the reversed low-storage Runge-Kutta recurrences, in place
+ * (the transpose of hedge/timestep/runge_kutta.py:123-128), FP64:
+ *   lam <- lam + b lq;   lq <- lq + dt (dR/dq)^T lam;
+ *   c_bar <- c_bar + dt (dR/dc)^T lam  (unless NULL);   lam <- a lam
+ * with lam, lq [F][K*Np], c_bar [K*Np] and the other arguments as in
+ * hb_rhs_adjoint; none of lam, lq and q may overlap.  Orders 1 to 7, else
+ * HB_ERR_UNSUPPORTED (compose the stage from hb_rhs_adjoint). */
+hb_status hb_adjoint_stage(hb_op* op, double a, double b, double dt, const double* q,
+                           double* lam, double* lq, double* c_bar, const double* coeff,
+                           void* work, void* stream);
+
 /* Batched ensemble: one launch per LSRK stage advances many independent
  * discretizations of uneven size and order.  Each member is a compiled
  * operator (advection or constant-c wave, HB_PREC_FP32, no given boundary
