@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhedge_b200.so")
 SOURCES = ["api.cu", "rhs_simt.cu", "rhs_split.cu", "norm.cu", "adjoint.cu", "ensemble.cu",
-           "waitcheck.cu", "rhs_quad.cu"]
+           "waitcheck.cu", "rhs_quad.cu", "quad_fp64.cu"]
 # the FP64 tensor-core kernels' instances, in parts that compile side by side:
 # (source, macro that selects the part, parts)
 PARTS = [("rhs_fp64.cu", "HB_FP64_PART", 5), ("adjoint_fp64.cu", "HB_ADJ_PART", 4)]

@@ -92,7 +92,7 @@ hb_status launch_wait_selftest(int* err, uint64_t limit_ns, cudaStream_t s);
 // The quadrature matrices in the kernel's layouts (each transposed so that
 // consecutive threads read consecutive entries): It [np][nq],
 // Bt [dim][nq][np], Ft [nf][nfp][nqf], Lt [nf*nqf][np], back to back; FP32
-// copies for FP32 operators; the element-maximum buffer for the LF flux.
+// copies for FP32 operators.
 static hb_status upload_quadrature(Op* op, const hb_quad_desc* qd) {
   const Discr* d = op->d;
   const int np = d->np, nfp = d->nfp, nf = d->nfaces, dim = d->dim;
@@ -118,12 +118,8 @@ static hb_status upload_quadrature(Op* op, const hb_quad_desc* qd) {
     if (!std::isfinite(x)) return fail(HB_ERR_INVALID_ARGUMENT, "non-finite quadrature matrix");
   op->nq = nq;
   op->nqf = nqf;
-  hb_status st;
   // FP64 matrices for both precisions (the FP32 path computes in FP64)
-  if ((st = upload(&op->quad64, h.data(), h.size()))) return st;
-  if (cudaMalloc(&op->elmax, sizeof(double) * d->K) != cudaSuccess)
-    return fail(HB_ERR_CUDA, "cannot allocate the element maxima");
-  return HB_OK;
+  return upload(&op->quad64, h.data(), h.size());
 }
 
 }  // namespace hb
@@ -291,7 +287,7 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
   hb_status st;
   auto bail = [&](hb_status s) {
     cudaFree(op->conn); cudaFree(op->err_flag);
-    cudaFree(op->quad64); cudaFree(op->elmax); cudaFree(op->afrag); cudaFree(op->adjfrag);
+    cudaFree(op->quad64); cudaFree(op->quadfrag); cudaFree(op->elmax); cudaFree(op->afrag); cudaFree(op->adjfrag);
     free_split(op);
     delete op;
     return s;
@@ -303,8 +299,14 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
     return bail(fail(HB_ERR_CUDA, "cannot allocate the device error flag"));
   if (op->precision == HB_PREC_FP32 && (st = ensure_fp32(d))) return bail(st);
   if (model == HB_MODEL_VARADV) {
-    st = upload_quadrature(op, qd);
-    if (!st) st = prepare_quad(op);
+    // buffer of the element maxima the LF flux reads
+    if (cudaMalloc(&op->elmax, sizeof(double) * d->K) != cudaSuccess)
+      return bail(fail(HB_ERR_CUDA, "cannot allocate the element maxima"));
+    st = prepare_quad_f64(op, qd);
+    if (st == HB_ERR_UNSUPPORTED) {
+      st = upload_quadrature(op, qd);
+      if (!st) st = prepare_quad(op);
+    }
   } else if (op->precision == HB_PREC_BF16X3 || op->precision == HB_PREC_FP16X3) {
     st = prepare_split(op);
     op->split = 1;
@@ -336,7 +338,7 @@ hb_status hb_op_destroy(hb_op* handle) {
   DeviceGuard g(op->d->device);
   cudaFree(op->conn);
   cudaFree(op->err_flag);
-  cudaFree(op->quad64); cudaFree(op->elmax); cudaFree(op->afrag); cudaFree(op->adjfrag);
+  cudaFree(op->quad64); cudaFree(op->quadfrag); cudaFree(op->elmax); cudaFree(op->afrag); cudaFree(op->adjfrag);
   free_split(op);
   delete op;
   return HB_OK;

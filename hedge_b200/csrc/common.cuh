@@ -109,6 +109,7 @@ struct Op {
   // element maxima of |v|^2 the LF flux reads
   int nq = 0, nqf = 0;
   double* quad64 = nullptr;
+  double* quadfrag = nullptr;  // the same in FP64 matrix fragments (quad_fp64.cu)
   double* elmax = nullptr;
 };
 
@@ -156,6 +157,11 @@ hb_status prepare_f64(Op* op);
 
 // quadrature kernel (rhs_quad.cu); vel = the velocity field [dim][K*Np]
 hb_status prepare_quad(Op* op);
+// its FP64 tensor-core form (quad_fp64.cu), for the element sizes built
+hb_status prepare_quad_f64(Op* op, const hb_quad_desc* qd);
+hb_status launch_quad_f64(Op* op, int mode, double ra, double rb, double dt, const void* q_in,
+                          void* q_out, void* res, const double* vel, const double* bdry,
+                          cudaStream_t s);
 hb_status launch_quad(Op* op, int mode, double ra, double rb, double dt, const void* q_in,
                       void* q_out, void* res, const double* vel, const double* bdry,
                       cudaStream_t s);

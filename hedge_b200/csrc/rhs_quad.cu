@@ -15,7 +15,9 @@
 // projection matrices; |J| cancels against the element Jacobian of the
 // integrals, and the face integrals carry Fscale = face Jacobian / |J|.
 //
-// One persistent CTA of 256 threads loops over batches of E elements:
+// This file's kernel runs on the CUDA cores, for the element sizes that the
+// FP64 tensor-core form (quad_fp64.cu) is not built for.  One persistent CTA
+// of 256 threads loops over batches of E elements:
 //   A. stage u and v (all components) of the batch in shared memory
 //      (coalesced), the geometry and the face table;
 //   B. gather the other side's u and v at every face node (the matched
@@ -409,11 +411,6 @@ static hb_status quad_launch(Op* op, int mode, double ra, double rb, double dt,
     op->grid = (int)std::min<int64_t>(nbatch, (int64_t)sms * per_sm);
     return HB_OK;
   }
-  if (op->mp.flux_type == 2) {
-    const int grid = (int)std::min<int64_t>((d->K + 255) / 256, 148 * 8);
-    elmax_kernel<<<grid, 256, 0, s>>>(d->K, d->np, d->dim, vel, op->elmax);
-    HB_CUDA(cudaGetLastError());
-  }
   QuadArgs<T, IO> a;
   a.K = d->K;
   a.E = op->elems_per_block;
@@ -468,6 +465,14 @@ hb_status prepare_quad(Op* op) {
 hb_status launch_quad(Op* op, int mode, double ra, double rb, double dt, const void* q_in,
                       void* q_out, void* res, const double* vel, const double* bdry,
                       cudaStream_t s) {
+  if (op->mp.flux_type == 2) {
+    const Discr* d = op->d;
+    const int grid = (int)std::min<int64_t>((d->K + 255) / 256, 148 * 8);
+    elmax_kernel<<<grid, 256, 0, s>>>(d->K, d->np, d->dim, vel, op->elmax);
+    HB_CUDA(cudaGetLastError());
+  }
+  if (op->quadfrag)
+    return launch_quad_f64(op, mode, ra, rb, dt, q_in, q_out, res, vel, bdry, s);
   if (op->precision == HB_PREC_FP32)
     return quad_dispatch<double, float>(op, mode, ra, rb, dt, q_in, q_out, res, vel, bdry, s,
                                         false);
