@@ -23,7 +23,7 @@ from __future__ import annotations
 
 import numpy as np
 
-from .timestep import RK4A, RK4B, RK4C
+from .timestep import _A, _B, RK4A, RK4B, RK4C
 
 
 def _torch():
@@ -126,25 +126,29 @@ class ReceiverTraces:
     _fn = None
 
     @staticmethod
-    def _stage_source(source, t):
+    def _amplitudes(source, dt, nsteps, device):
+        """[nsteps, 5] source amplitudes at the stage times, on the device."""
         if source is None:
             return None
-        vec, amp = source
-        return vec * float(amp(t))
+        t, rows = 0.0, []
+        for _ in range(nsteps):
+            rows.append([float(source[1](t + cs * dt)) for cs in RK4C])
+            t += dt
+        return _torch().tensor(rows, dtype=_torch().float64, device=device)
 
-    @classmethod
-    def _step(cls, comp, q, res, c, dt, t, source, keep=None):
-        torch = _torch()
-        cur = q
-        for s in range(5):
-            a, b, cs = RK4A[s], RK4B[s], RK4C[s]
-            if keep is not None:
-                keep.append(cur)
-            nxt = torch.empty_like(cur)
-            comp.lsrk_stage(a, b, dt, cur, nxt, res, coeff=c,
-                            source=cls._stage_source(source, t + cs * dt))
-            cur = nxt
-        return cur
+    @staticmethod
+    def _step(comp, bufs, res, c, dt, source, amps):
+        """One step through the stage buffers bufs[0] -> .. -> bufs[5]."""
+        if source is None:
+            comp.lsrk_step(_A, _B, dt, bufs, res, coeff=c)
+        elif comp.var_material:
+            for s in range(5):
+                comp.lsrk_stage(RK4A[s], RK4B[s], dt, bufs[s], bufs[s + 1], res, coeff=c,
+                                source=source[0] * amps[s])
+        else:
+            src = amps[:, None] * source[0].reshape(1, -1)
+            comp.lsrk_step(_A, _B, dt, bufs, res, coeff=c, source=src,
+                           source_stride=src.shape[1])
 
     @classmethod
     def apply(cls, q0, c, comp, receivers, dt, nsteps, source=None, checkpoint_every=20):
@@ -159,16 +163,24 @@ class ReceiverTraces:
                     res = torch.zeros_like(q)
                     traces = [receivers(q)]
                     checkpoints = {0: q}
-                    t = 0.0
+                    if source is not None and not comp.var_material:
+                        # a stage's source is amplitude * vector: refuse a
+                        # vector whose products the kernels cannot read
+                        comp._field_ptrs(cc, torch.empty_like(source[0]))
+                    amps = cls._amplitudes(source, dt, nsteps, q.device)
+                    tmp = [torch.empty_like(q), torch.empty_like(q)]
                     for n in range(nsteps):
-                        q = cls._step(comp, q, res, cc, dt, t, source)
-                        t += dt
+                        bufs = [q, tmp[0], tmp[1], tmp[0], tmp[1], torch.empty_like(q)]
+                        cls._step(comp, bufs, res, cc, dt, source,
+                                  None if amps is None else amps[n])
+                        q = bufs[5]
                         traces.append(receivers(q))
                         if (n + 1) % every == 0 and n + 1 < nsteps:
                             checkpoints[n + 1] = q
                     ctx.comp, ctx.receivers, ctx.dt, ctx.nsteps = comp, receivers, dt, nsteps
                     ctx.source, ctx.every, ctx.checkpoints = source, every, checkpoints
                     ctx.has_c = cc is not None
+                    ctx.amps = amps
                     ctx.save_for_backward(cc if cc is not None else torch.empty(0))
                     return torch.stack(traces)
 
@@ -188,12 +200,13 @@ class ReceiverTraces:
                         q = ctx.checkpoints[s0]
                         res = torch.zeros_like(q)
                         stages = []
-                        t = s0 * dt
                         for n in range(s0, s1):
-                            keep = []
-                            q = cls._step(comp, q, res, cc, dt, t, ctx.source, keep)
-                            stages.append(keep)
-                            t += dt
+                            out = torch.empty((5,) + q.shape, dtype=q.dtype, device=q.device)
+                            bufs = [q, *out]
+                            cls._step(comp, bufs, res, cc, dt, ctx.source,
+                                      None if ctx.amps is None else ctx.amps[n])
+                            stages.append(bufs[:5])
+                            q = bufs[5]
                         # reverse through the segment
                         for n in range(s1 - 1, s0 - 1, -1):
                             keep = stages[n - s0]

@@ -411,6 +411,25 @@ hb_status hb_lsrk_stage(hb_op* handle, double a, double b, double dt, const void
   return run(op, 1, a, b, dt, q_in, q_out, res, coeff, bdry, source, stream);
 }
 
+hb_status hb_lsrk_step(hb_op* handle, int32_t n, const double* a, const double* b, double dt,
+                       void* const* q, void* res, const double* coeff, const double* bdry,
+                       const double* source, int64_t source_stride, void* stream) {
+  if (!handle) return fail(HB_ERR_INVALID_ARGUMENT, "null operator");
+  if (n < 1 || !a || !b || !q) return fail(HB_ERR_INVALID_ARGUMENT, "null or empty stage list");
+  Op* op = reinterpret_cast<Op*>(handle);
+  for (int s = 0; s < n; ++s) {
+    const hb_status st = check_inputs(op, q[s], q[s + 1], coeff, bdry);
+    if (st) return st;
+  }
+  if (!res) return fail(HB_ERR_INVALID_ARGUMENT, "null residual pointer");
+  for (int s = 0; s < n; ++s) {
+    const hb_status st = run(op, 1, a[s], b[s], dt, q[s], q[s + 1], res, coeff, bdry,
+                             source ? source + s * source_stride : nullptr, stream);
+    if (st) return st;
+  }
+  return HB_OK;
+}
+
 hb_status hb_rhs_elements(hb_op* handle, int64_t el_begin, int64_t el_end, const void* q,
                           void* rhs, const double* coeff, const double* bdry,
                           const double* source, void* stream) {

@@ -25,7 +25,7 @@ from .lowering import as_descriptor
 from .optemplate import Expr
 from .models import (BC_GIVEN, BC_INCIDENT, BC_NONE, MODEL_MAXWELL, MODEL_MAXWELL_TE,
                      MODEL_MAXWELL_TM, MODEL_VARADV, MODEL_VARWAVE, MODEL_WAVE,
-                     MODEL_ADVECTION, OpTemplate)
+                     MODEL_ADVECTION, OpTemplate, TimeConstantGivenFunction)
 from .quadrature import ElementQuadrature
 from .refelem import make_element
 
@@ -696,6 +696,22 @@ class CompiledOperator:
             self._handle, float(a), float(b), float(dt), q_in.data_ptr(),
             q_out.data_ptr(), res.data_ptr(), cptr, bptr, sptr, self._stream()))
 
+    def lsrk_step(self, a, b, dt, bufs, res, bc_in=None, coeff=None, source=None,
+                  source_stride=0):
+        """Stages bufs[s] -> bufs[s + 1] with coefficients a[s], b[s] (ctypes
+        arrays of doubles) in one native call; boundary values, coefficient
+        and, unless ``source_stride`` (values between the stages' sources)
+        is given, source hold for all of them."""
+        keep, bptr = self._bdry_ptr(bc_in)
+        if source_stride:
+            cptr, sptr = self._field_ptrs(coeff, None)[0], source.data_ptr()
+        else:
+            cptr, sptr = self._field_ptrs(coeff, source)
+        _native.check(self._lib.hb_lsrk_step(
+            self._handle, len(a), a, b, float(dt),
+            (C.c_void_p * len(bufs))(*[x.data_ptr() for x in bufs]), res.data_ptr(), cptr, bptr,
+            sptr, source_stride, self._stream()))
+
     def adjoint(self, lam, q=None, coeff=None, want_c=False):
         """Adjoint of the RHS (hb_rhs_adjoint), FP64: returns
         (q_bar, c_bar) = ((dR/dq)^T lam, (dR/dc)^T lam at the state q).
@@ -865,6 +881,18 @@ class BoundRHS:
             if hasattr(m, "context"):
                 return m.context(self.discr, t)
         return {}
+
+    def constant_context(self):
+        """Whether ``context`` is the same at all times: the model has no
+        boundary data or velocity to evaluate, or gives them as
+        TimeConstantGivenFunctions."""
+        comp = self.compiled
+        if not comp.n_given and comp.ot.model != MODEL_VARADV:
+            return True
+        given = [getattr(self.model, n, None)
+                 for n in ("inflow_u", "dirichlet_bc_f", "advec_v", "bc_u_f")]
+        return all(x is None or isinstance(x, str) or type(x) is TimeConstantGivenFunction
+                   for x in given)
 
     def __call__(self, t, w, **extra_context):
         kw = self.context(t)

@@ -9,6 +9,8 @@ linear combiner does (hedge/vector_primitives.py:58-77).
 
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 
 from . import _native
@@ -28,6 +30,9 @@ RK4C = [0.0,
         2526269341429 / 6820363962896,
         2006345519317 / 3224310063776,
         2802321613138 / 2924317926251]
+
+# the same for the native step
+_A, _B = (C.c_double * 5)(*RK4A), (C.c_double * 5)(*RK4B)
 
 
 class LSRK4TimeStepper:
@@ -50,6 +55,11 @@ class LSRK4TimeStepper:
             # ping-pong between two fresh buffers; the caller's y is not
             # written (the reference also returns a new state each step)
             bufs = [torch.empty_like(y), torch.empty_like(y)]
+            if rhs.constant_context():
+                # the model's data evaluated once, the five stages in one call
+                comp.lsrk_step(_A, _B, dt, [y, bufs[0], bufs[1], bufs[0], bufs[1], bufs[0]],
+                               self.residual, **rhs.context(t))
+                return bufs[0]
             cur = y
             for s, (a, b, c) in enumerate(self.coeffs):
                 nxt = bufs[s % 2]

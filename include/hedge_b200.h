@@ -167,6 +167,15 @@ hb_status hb_lsrk_stage(hb_op* op, double a, double b, double dt,
                         const double* coeff, const double* bdry,
                         const double* source, void* stream);
 
+/* n consecutive stages (a step) in one call, as n calls of hb_lsrk_stage:
+ * stage s reads q[s] and writes q[s + 1] (n + 1 device pointers in a host
+ * array, neighbours distinct; a buffer may return later in the list) with
+ * coefficients a[s], b[s].  coeff and bdry hold for all stages; stage s takes
+ * source + s * source_stride (in values; 0: the same source). */
+hb_status hb_lsrk_step(hb_op* op, int32_t n, const double* a, const double* b, double dt,
+                       void* const* q, void* res, const double* coeff, const double* bdry,
+                       const double* source, int64_t source_stride, void* stream);
+
 /* hb_rhs / hb_lsrk_stage for the elements [el_begin, el_end) of the
  * operator's K only (the other elements' outputs are left as they are; the
  * inputs are the whole [F][K*Np] vectors).  They split one stage of an
