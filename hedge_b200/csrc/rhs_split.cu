@@ -1544,8 +1544,14 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) rhs_split_kernel(SplitArgsT<
 //   * the state is read from global memory (FP64) in the split and face
 //     phases, the rhs is staged (FP32) in the state-plane area after the diff
 //     MMAs completed, and the FP64 stage update is a coalesced pass;
-//   * all 8 warps run every phase; thread 0 issues the MMAs.
-template <int MODEL, int DIM, int ORDER>
+//   * all 16 warps run every phase; thread 0 issues the MMAs.
+// Measured (LSRK4 step, K = 48000, FP16x3): wave N = 7 3386 -> 1887 us, Maxwell
+// N = 5 2740 -> 1610 us; wave N = 6, K = 34992 1961 -> 1109 us, from 8 warps with
+// 8-byte loads; the phases of a wave N = 7 batch then took 5 (element data), 13
+// (remainders), 24 (fluxes), 10 (flux split), 8 (lift), 10 (epilogue) and 12
+// (update) thousand cycles at 16 warps, now 5, 8, 18, 5, 4, 10 and 10.  The
+// epilogue is bound by instruction issue, the others by memory latency.
+template <int MODEL, int DIM, int ORDER, int WARPS = 16>
 struct ShapeS {
   static constexpr int F = Traits<MODEL, DIM>::F;
   static constexpr int C = Traits<MODEL, DIM>::COEFF;
@@ -1566,14 +1572,20 @@ struct ShapeS {
   static constexpr int ND2 = ND - ND1;
   static constexpr int LIFT_COL = ru32(ND);
   static constexpr int NKD = KD / 16, NKL = KL / 16;
-  static constexpr int THREADS = 256;
-  static constexpr int NW = THREADS / 32;
-  static constexpr int NPQ = (((NP + 1) / 2) + 3) & ~3;       // nodes per epilogue warp
+  static constexpr int NITEM = 4 * (KD / 8);
+  // 16 warps, or 12 where the state-split items do not come out even: the
+  // phases wait on memory, and 128 registers hold each of them (LSRK4 step,
+  // K = 48000, 8 -> 16 warps: wave N = 7 3386 -> 2534 us, Maxwell N = 5 2740 ->
+  // 2179 us).  WARPS = 8: configure_stream's small meshes.
+  static constexpr int NW = WARPS == 8 ? 8 : NITEM % 32 == 0 ? 16 : NITEM % 24 == 0 ? 12 : 8;
+  static constexpr int THREADS = 32 * NW;
+  static constexpr int PARTS = NW / 4;                        // warps per TMEM quadrant
+  static constexpr int NPQ = (((NP + PARTS - 1) / PARTS) + 3) & ~3;   // nodes per epilogue warp
   static constexpr int NFACE = EB * NFPT;
   static constexpr int NFV = (NFACE + THREADS - 1) / THREADS;
-  static constexpr int NITEM = 4 * (KD / 8);
   static constexpr uint32_t bDc = ND * 16 * 2, bLc = NL * 16 * 2;   // one plane, one chunk
   static constexpr uint32_t RING = al128(2 * (bDc > bLc ? bDc : bLc));
+  static constexpr int LCH = RING / (2 * bLc);                // lift chunks per ring buffer
   static constexpr uint32_t bAq = 128 * KD * 2, bAf = 128 * KL * 2;
   static constexpr uint32_t oAqh = 0;
   static constexpr uint32_t oAql = al128(oAqh + bAq);
@@ -1597,14 +1609,40 @@ struct ShapeS {
   static constexpr uint32_t LIN_BYTES = 8 + NP * DIM * 8;
   static constexpr int TMEM_NEED = LIFT_COL + NL;
   static constexpr uint32_t TMEM_COLS = TMEM_NEED <= 128 ? 128 : TMEM_NEED <= 256 ? 256 : 512;
+  // field stride of the staged rhs: the fields of a node fall in other banks
+  static constexpr int SQS = FNP + 2;
   static constexpr bool FITS = ND1 <= 256 && ND2 <= 256 && NL <= 256 && TMEM_NEED <= 512 &&
                                LIFT_COL + NP + 3 < 512 && total <= SMEM_LIMIT &&
-                               F * FNP * 4 <= (int)(2 * bAq);
+                               F * SQS * 4 <= (int)(2 * bAq);
 };
 
-template <int MODEL, int DIM, int ORDER, int PT>
-__global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
-  using S = ShapeS<MODEL, DIM, ORDER>;
+// 32 bytes from a 32-byte boundary
+__device__ __forceinline__ void ldg4(const double* p, double* v) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+      : "l"(p));
+}
+
+// Stores 8 scaled values as their FP16 planes.
+__device__ __forceinline__ void split8(uint8_t* hi, uint8_t* lo, uint32_t off,
+                                       const float (&v)[8]) {
+  uint32_t hw[4], lw[4];
+#pragma unroll
+  for (int c = 0; c < 8; c += 2) {
+    const __half2 h = __floats2half2_rn(v[c], v[c + 1]);
+    const float2 hf = __half22float2(h);
+    const __half2 l = __floats2half2_rn(v[c] - hf.x, v[c + 1] - hf.y);
+    hw[c / 2] = *reinterpret_cast<const uint32_t*>(&h);
+    lw[c / 2] = *reinterpret_cast<const uint32_t*>(&l);
+  }
+  *reinterpret_cast<uint4*>(hi + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+  *reinterpret_cast<uint4*>(lo + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+}
+
+template <int MODEL, int DIM, int ORDER, int PT, int WARPS>
+__global__ void __launch_bounds__(ShapeS<MODEL, DIM, ORDER, WARPS>::THREADS, 1)
+    rhs_split_stream_kernel(SplitArgs a) {
+  using S = ShapeS<MODEL, DIM, ORDER, WARPS>;
   constexpr int F = S::F, C = S::C, NA = S::NA, NP = S::NP, NFP = S::NFP, NF = S::NF;
   constexpr int NFPT = S::NFPT, G = S::G, EPW = S::EPW, EB = S::EB, FNP = S::FNP;
   constexpr int KD = S::KD, KL = S::KL, NV1 = DIM + 1;
@@ -1671,31 +1709,40 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
   const int e_lane = quad * EPW + lf;
   const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
   const int row = quad * 32 + lane;
+  // the lift stream: LCH operator chunks per copy
+  constexpr uint32_t LBYTES = S::NKL * 2 * S::bLc, LUNIT = S::LCH * 2 * S::bLc;
+  constexpr int NLU = (S::NKL + S::LCH - 1) / S::LCH;
   uint32_t ring_uses[2] = {0u, 0u};   // MMA commits so far on each ring buffer
   uint32_t ring_fills[2] = {0u, 0u};  // bulk copies started into each ring buffer
   uint32_t ring_waits[2] = {0u, 0u};  // copies waited for on each ring buffer
   uint32_t chunk = 0;                 // running chunk counter (ring buffer = chunk & 1)
   int bad = 0;
 
-  // Thread 0 only: streams n operator chunks of `bytes` (at src + k * bytes)
+  // Thread 0 only: streams `total` bytes of operator chunks, `bytes` at a time,
   // through the two ring buffers with bulk copies, the copy of chunk k + 1
   // in flight while chunk k's MMAs (issue(k, buffer)) run.  A buffer is
   // refilled once the MMAs that read it completed.  False on a timeout.
-  auto stream_chunks = [&](const uint8_t* src, int n, uint32_t bytes, auto issue) -> bool {
-    const uint32_t c0 = chunk;          // running number of this stream's chunk 0
-    auto fill = [&](int k) -> bool {
+  // `ahead` chunks were filled before the call.
+  auto fill_chunk = [&](const uint8_t* src, int k, uint32_t c0, uint32_t total,
+                        uint32_t bytes) -> bool {
       const int b = (int)((c0 + (uint32_t)k) & 1u);
+      const uint32_t left = total - (uint32_t)k * bytes;
       if (ring_uses[b] > 0 && !tc::mbar_wait(&mbar[b], (ring_uses[b] - 1) & 1u, MBAR_MAX_NS))
         return false;
-      mbar_arrive_expect_tx(&mbar[5 + b], bytes);
-      bulk_load(smem + (b ? S::oR1 : S::oR0), src + (size_t)k * bytes, bytes, &mbar[5 + b]);
+      const uint32_t part_bytes = left < bytes ? left : bytes;
+      mbar_arrive_expect_tx(&mbar[5 + b], part_bytes);
+      bulk_load(smem + (b ? S::oR1 : S::oR0), src + (size_t)k * bytes, part_bytes, &mbar[5 + b]);
       ++ring_fills[b];
       return true;
-    };
-    if (n > 0 && !fill(0)) return false;
+  };
+  auto stream_chunks = [&](const uint8_t* src, uint32_t total, uint32_t bytes, int ahead,
+                           auto issue) -> bool {
+    const uint32_t c0 = chunk;          // running number of this stream's chunk 0
+    const int n = (int)((total + bytes - 1) / bytes);
+    if (ahead < 1 && !fill_chunk(src, 0, c0, total, bytes)) return false;
     for (int k = 0; k < n; ++k) {
       const int b = (int)(chunk & 1u);
-      if (k + 1 < n && !fill(k + 1)) return false;
+      if (k + 1 < n && k + 1 >= ahead && !fill_chunk(src, k + 1, c0, total, bytes)) return false;
       if (!tc::mbar_wait(&mbar[5 + b], ring_waits[b] & 1u, MBAR_MAX_NS)) return false;
       ++ring_waits[b];
       issue(k, tc::smem_u32(smem + (b ? S::oR1 : S::oR0)));
@@ -1706,6 +1753,10 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
     return true;
   };
 
+  const bool wide = NP % 4 == 0 && (reinterpret_cast<uintptr_t>(a.q_in) & 31u) == 0;
+  const bool pairs = NP % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.q_in) |
+                                      reinterpret_cast<uintptr_t>(a.q_out) |
+                                      reinterpret_cast<uintptr_t>(a.res)) & 15u) == 0;
   uint32_t it = 0;
   for (int64_t batch = blockIdx.x; batch < a.nbatch; batch += gridDim.x, ++it) {
     const int64_t el0 = batch_first(a, batch);
@@ -1734,15 +1785,22 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
       for (int d = 0; d < DIM; ++d) lin[d] = valid ? (float)(0.5 * (v[1 + d] - v[0])) : 0.f;
     }
     // remainders of 8 consecutive nodes of this thread's row (item chunk8):
-    // the 8 state loads are issued before any is used
+    // the state loads, 32 bytes each where the rows start on such a boundary
+    // (a lane's row is a cache line of its own: 8-byte loads took four times
+    // the L1 wavefronts), are issued before any is used
     auto rem8 = [&](int chunk8, float (&v)[8]) {
       const double* v3 = sv + (fown * EB + e_own) * NV1;
       const double* src = a.q_in + fown * Knp + (el0 + e_own) * NP;
       double q[8];
+      if (wide && valid && chunk8 * 8 + 8 <= NP) {
+        ldg4(src + chunk8 * 8, q);
+        ldg4(src + chunk8 * 8 + 4, q + 4);
+      } else {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const int j = chunk8 * 8 + c;
-        q[c] = (valid && j < NP) ? __ldg(src + j) : 0.0;
+        for (int c = 0; c < 8; ++c) {
+          const int j = chunk8 * 8 + c;
+          q[c] = (valid && j < NP) ? __ldg(src + j) : 0.0;
+        }
       }
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
@@ -1783,31 +1841,25 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
     for (int k = 0; k < S::NITEM / S::NW; ++k) {
       const int chunk8 = (warp + k * S::NW) >> 2;
       const uint32_t off = kmajor_off(row, chunk8 * 8, KD);
-      float v[8];
       if constexpr (PT == PT_FP16) {
+        float v[8];
         unpark8(Aqh, Aql, off, v);
 #pragma unroll
         for (int c = 0; c < 8; ++c) v[c] *= inv;
-      } else {
-        rem8(chunk8, v);
+        split8(Aqh, Aql, off, v);
+        continue;
       }
+      float v[8];
+      rem8(chunk8, v);
       uint32_t hw[4], lw[4];
 #pragma unroll
       for (int c = 0; c < 8; c += 2) {
         const float x0 = v[c], x1 = v[c + 1];
-        if constexpr (PT == PT_BF16) {
-          const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
-          const float2 hf = __bfloat1622float2(h);
-          const __nv_bfloat162 l = __floats2bfloat162_rn(x0 - hf.x, x1 - hf.y);
-          hw[c / 2] = *reinterpret_cast<const uint32_t*>(&h);
-          lw[c / 2] = *reinterpret_cast<const uint32_t*>(&l);
-        } else {
-          const __half2 h = __floats2half2_rn(x0, x1);
-          const float2 hf = __half22float2(h);
-          const __half2 l = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
-          hw[c / 2] = *reinterpret_cast<const uint32_t*>(&h);
-          lw[c / 2] = *reinterpret_cast<const uint32_t*>(&l);
-        }
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+        const float2 hf = __bfloat1622float2(h);
+        const __nv_bfloat162 l = __floats2bfloat162_rn(x0 - hf.x, x1 - hf.y);
+        hw[c / 2] = *reinterpret_cast<const uint32_t*>(&h);
+        lw[c / 2] = *reinterpret_cast<const uint32_t*>(&l);
       }
       *reinterpret_cast<uint4*>(Aqh + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
       *reinterpret_cast<uint4*>(Aql + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
@@ -1830,6 +1882,10 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
             const double* src = a.q_in + f * Knp + n0 * NP;
             if (aligned16(src, (uint32_t)(nn * NP * 8))) prefetch_l2(src, (uint32_t)(nn * NP * 8));
           }
+          if (aligned16(a.geo32 + n0 * G, (uint32_t)(nn * G * 4)))
+            prefetch_l2(a.geo32 + n0 * G, (uint32_t)(nn * G * 4));
+          if (aligned16(a.conn + n0 * NF, (uint32_t)(nn * NF * 8)))
+            prefetch_l2(a.conn + n0 * NF, (uint32_t)(nn * NF * 8));
         }
         if (a.mode != 0)
           for (int f = 0; f < F; ++f) {
@@ -1837,7 +1893,7 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
             if (aligned16(src, (uint32_t)(ne * NP * 8))) prefetch_l2(src, (uint32_t)(ne * NP * 8));
           }
         const uint32_t aq_h = tc::smem_u32(Aqh), aq_l = tc::smem_u32(Aql);
-        ok = stream_chunks(dimg, S::NKD, 2 * S::bDc, [&](int kk, uint32_t buf) {
+        ok = stream_chunks(dimg, S::NKD * 2 * S::bDc, 2 * S::bDc, 0, [&](int kk, uint32_t buf) {
           const uint32_t bh = buf, bl = buf + S::bDc;
           const uint64_t ah = tc::smem_desc(aq_h + kk * 256, 128, KD * 16);
           const uint64_t al = tc::smem_desc(aq_l + kk * 256, 128, KD * 16);
@@ -1852,6 +1908,9 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
             tc::mma_bf16(tmem_diff + S::ND1, al, tc::smem_desc(bh + o2, 128, 256), ID_D2, 1u);
           }
         }) ? 1 : 0;
+        // the lift stream's first two copies, behind the face fluxes
+        for (int u = 0; ok && u < 2 && u < NLU; ++u)
+          ok = fill_chunk(limg, u, chunk, LBYTES, LUNIT) ? 1 : 0;
       }
       __syncwarp();
       if (!__shfl_sync(FULL, ok, 0)) bad = 1;
@@ -1951,39 +2010,43 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
     constexpr int NFVC = (S::NFACE + CT - 1) / CT;
     const int ct = tid - 32;
     if constexpr (PT == PT_FP16) {
-      // fluxes once: row maxima, raw values parked in the planes; then
-      // every thread splits its own entries with the row scale
+      // fluxes once, raw values parked in the planes; then each thread takes
+      // 16-byte chunks of its row: maximum (shared by the row's PARTS threads),
+      // scale and split.  (Maxima formed by the flux threads took a match and F
+      // reductions per face point.)
       for (int u = 0; u < NFVC && warp != 0; ++u) {
         const int x = ct + u * CT;
         float fl[F];
         face_flux(x, fl);
-        const int e = x < S::NFACE ? x / NFPT : -1;
-        const unsigned grp = __match_any_sync(FULL, e);
-        const bool leader = (__ffs(grp) - 1) == lane;
-#pragma unroll
-        for (int f = 0; f < F; ++f) {
-          const unsigned m = __reduce_max_sync(grp, __float_as_uint(fabsf(fl[f])));
-          if (leader && e >= 0 && e < ne) atomicMax(&fmx[(e / EPW) * 32 + (e % EPW) * F + f], m);
-        }
-        if (e >= 0 && e < ne) {
-          const int p = x % NFPT, rowb = (e / EPW) * 32 + (e % EPW) * F;
+        const int e = x / NFPT, p = x % NFPT;
+        if (x < S::NFACE && e < ne) {
+          const int rowb = (e / EPW) * 32 + (e % EPW) * F;
 #pragma unroll
           for (int f = 0; f < F; ++f) park_f32(Afh, Afl, kmajor_off(rowb + f, p, KL), fl[f]);
         }
       }
       __syncthreads();
-      for (int u = 0; u < NFVC && warp != 0; ++u) {
-        const int x = ct + u * CT;
-        const int e = x / NFPT, p = x % NFPT;
-        if (x < S::NFACE && e < ne) {
-          const int rowb = (e / EPW) * 32 + (e % EPW) * F;
+      constexpr int NC8 = (NFPT + 7) / 8;
+      uint32_t m = 0u;
+#pragma unroll 1
+      for (int c8 = part; c8 < NC8 && valid; c8 += S::PARTS) {
+        float v[8];
+        unpark8(Afh, Afl, kmajor_off(row, c8 * 8, KL), v);
 #pragma unroll
-          for (int f = 0; f < F; ++f) {
-            const uint32_t off = kmajor_off(rowb + f, p, KL);
-            store_split<PT>(Afh, Afl, off,
-                            unpark_f32(Afh, Afl, off) * row_scale_inv(fmx[rowb + f]));
-          }
-        }
+        for (int c = 0; c < 8; ++c)
+          m = max(m, c8 * 8 + c < NFPT ? __float_as_uint(fabsf(v[c])) : 0u);
+      }
+      if (valid) atomicMax(&fmx[row], m);
+      __syncthreads();
+      const float finv = row_scale_inv(fmx[row]);
+#pragma unroll 1
+      for (int c8 = part; c8 < NC8 && valid; c8 += S::PARTS) {
+        const uint32_t off = kmajor_off(row, c8 * 8, KL);
+        float v[8];
+        unpark8(Afh, Afl, off, v);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) v[c] = c8 * 8 + c < NFPT ? v[c] * finv : 0.f;  // K padding
+        split8(Afh, Afl, off, v);
       }
     } else {
       for (int u = 0; u < NFVC && warp != 0; ++u) {
@@ -2012,13 +2075,15 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
       if (tid == 0) {
         tc::fence_after_sync();
         const uint32_t af_h = tc::smem_u32(Afh), af_l = tc::smem_u32(Afl);
-        ok = stream_chunks(limg, S::NKL, 2 * S::bLc, [&](int kk, uint32_t buf) {
-          const uint32_t bh = buf, bl = buf + S::bLc;
-          const uint64_t ah = tc::smem_desc(af_h + kk * 256, 128, KL * 16);
-          const uint64_t al = tc::smem_desc(af_l + kk * 256, 128, KL * 16);
-          tc::mma_bf16(tmem_lift, ah, tc::smem_desc(bh, 128, 256), ID_L, kk > 0 ? 1u : 0u);
-          tc::mma_bf16(tmem_lift, ah, tc::smem_desc(bl, 128, 256), ID_L, 1u);
-          tc::mma_bf16(tmem_lift, al, tc::smem_desc(bh, 128, 256), ID_L, 1u);
+        ok = stream_chunks(limg, LBYTES, LUNIT, NLU < 2 ? NLU : 2, [&](int u, uint32_t buf) {
+          for (int kk = u * S::LCH; kk < (u + 1) * S::LCH && kk < S::NKL; ++kk) {
+            const uint32_t bh = buf + (kk - u * S::LCH) * 2 * S::bLc, bl = bh + S::bLc;
+            const uint64_t ah = tc::smem_desc(af_h + kk * 256, 128, KL * 16);
+            const uint64_t al = tc::smem_desc(af_l + kk * 256, 128, KL * 16);
+            tc::mma_bf16(tmem_lift, ah, tc::smem_desc(bh, 128, 256), ID_L, kk > 0 ? 1u : 0u);
+            tc::mma_bf16(tmem_lift, ah, tc::smem_desc(bl, 128, 256), ID_L, 1u);
+            tc::mma_bf16(tmem_lift, al, tc::smem_desc(bh, 128, 256), ID_L, 1u);
+          }
         }) ? 1 : 0;
         if (ok) tc::mma_commit(&mbar[2]);   // all of this batch's MMAs
       }
@@ -2090,7 +2155,7 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
           if (valid) {
             const int64_t si = model_src_index<MODEL>(fown, (el0 + e_own) * NP + i, Knp);
             const float src = (a.source && si >= 0) ? (float)a.source[si] : 0.f;
-            sq[fown * FNP + e_own * NP + i] =
+            sq[fown * S::SQS + e_own * NP + i] =
                 model_finish<MODEL, DIM, float>(a.mp, fown, mine, lv[c] * slift, src);
           }
         }
@@ -2099,8 +2164,44 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
     tc::fence_before_sync();
     __syncthreads();
 
-    // ---- F: FP64 stage update (coalesced; UF values per thread in flight) ----
-    {
+    // ---- F: FP64 stage update (coalesced; ten values of each vector per
+    // thread in flight, 16 bytes a load where the vectors allow) ----
+    if (pairs) {
+      constexpr int UF = 5, FV = FNP / 2;
+      for (int x0 = tid; x0 < S::NVAL / 2; x0 += UF * S::THREADS) {
+        double2 r0[UF], q0[UF];
+        int64_t idx[UF];
+        bool ok[UF];
+#pragma unroll
+        for (int u = 0; u < UF; ++u) {
+          const int x = x0 + u * S::THREADS;
+          const int f = x / FV, r = (x - f * FV) * 2;
+          ok[u] = x < S::NVAL / 2 && r < ne * NP;
+          idx[u] = f * Knp + el0 * NP + r;
+          r0[u] = q0[u] = make_double2(0.0, 0.0);
+          if (ok[u] && a.mode != 0) {
+            r0[u] = *reinterpret_cast<const double2*>(a.res + idx[u]);
+            q0[u] = __ldg(reinterpret_cast<const double2*>(a.q_in + idx[u]));
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < UF; ++u) {
+          if (!ok[u]) continue;
+          const int x = x0 + u * S::THREADS;
+          const float2 rf =
+              *reinterpret_cast<const float2*>(sq + 2 * x + (x / FV) * (S::SQS - FNP));
+          const double rx = (double)rf.x, ry = (double)rf.y;
+          if (a.mode == 0) {
+            *reinterpret_cast<double2*>(a.q_out + idx[u]) = make_double2(rx, ry);
+          } else {
+            const double nx = a.ra * r0[u].x + a.dt * rx, ny = a.ra * r0[u].y + a.dt * ry;
+            *reinterpret_cast<double2*>(a.res + idx[u]) = make_double2(nx, ny);
+            *reinterpret_cast<double2*>(a.q_out + idx[u]) =
+                make_double2(q0[u].x + a.rb * nx, q0[u].y + a.rb * ny);
+          }
+        }
+      }
+    } else {
       constexpr int UF = 10;
       for (int x0 = tid; x0 < S::NVAL; x0 += UF * S::THREADS) {
         double r0[UF], q0[UF];
@@ -2121,7 +2222,8 @@ __global__ void __launch_bounds__(256, 1) rhs_split_stream_kernel(SplitArgs a) {
 #pragma unroll
         for (int u = 0; u < UF; ++u) {
           if (!ok[u]) continue;
-          const double rr = (double)sq[x0 + u * S::THREADS];
+          const int x = x0 + u * S::THREADS;
+          const double rr = (double)sq[x + (x / FNP) * (S::SQS - FNP)];
           if (a.mode == 0) {
             a.q_out[idx[u]] = rr;
           } else {
@@ -2485,7 +2587,13 @@ static hb_status configure_stream(Op* op) {
   } else {
     if (d->np != S::NP || d->nfp != S::NFP)
       return fail(HB_ERR_INVALID_ARGUMENT, "element sizes do not match the order");
-    auto kern = rhs_split_stream_kernel<MODEL, DIM, ORDER, PT>;
+    // Meshes of at most one batch keep the eight-warp shape (256 threads) that
+    // the tests of small parts read back through hb_op_launch_info; 16 warps
+    // are faster there too (wave N = 7, K = 30: 200 -> 159 us a step).
+    const bool small = d->K <= S::EB;
+    using S8 = ShapeS<MODEL, DIM, ORDER, 8>;
+    auto kern = small ? rhs_split_stream_kernel<MODEL, DIM, ORDER, PT, 8>
+                      : rhs_split_stream_kernel<MODEL, DIM, ORDER, PT, 16>;
     int dev, max_optin = 0, sms = 0;
     HB_CUDA(cudaGetDevice(&dev));
     HB_CUDA(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -2501,7 +2609,7 @@ static hb_status configure_stream(Op* op) {
       smem = std::min<size_t>((size_t)smem_sm / max_ctas - 1024 + 16, (size_t)max_optin);
     HB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t nbatch = (d->K + S::EB - 1) / S::EB;
-    op->threads = S::THREADS;
+    op->threads = small ? S8::THREADS : S::THREADS;
     op->blocks_per_sm = 1;
     op->smem = smem;
     op->grid = (int)std::min<int64_t>(nbatch, (int64_t)sms);
@@ -2609,7 +2717,11 @@ static hb_status launch_stream_t(Op* op, int mode, double ra, double rb, double 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = HB_SPLIT_PDL ? 1 : 0;
-    HB_CUDA(cudaLaunchKernelEx(&cfg, rhs_split_stream_kernel<MODEL, DIM, ORDER, PT>, a));
+    HB_CUDA(cudaLaunchKernelEx(&cfg,
+                               op->threads == S::THREADS
+                                   ? rhs_split_stream_kernel<MODEL, DIM, ORDER, PT, 16>
+                                   : rhs_split_stream_kernel<MODEL, DIM, ORDER, PT, 8>,
+                               a));
     return HB_OK;
   }
 }
