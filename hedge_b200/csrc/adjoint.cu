@@ -1,5 +1,6 @@
 // Adjoint (transpose) of the DG right-hand side, FP64, on the CUDA cores: the
-// orders beyond 7 (adjoint_fp64.cu serves 1 to 7).
+// orders beyond 7 (adjoint_fp64.cu serves 1 to 7), and an operator's first call
+// where that comes under stream capture.
 //
 // For R(q; c) as computed by hb_rhs (volume terms from the chain rule of the
 // reference derivatives, face fluxes lifted with LIFT and the inverse-Jacobian
@@ -339,7 +340,8 @@ int64_t adjoint_work_bytes(const Op* op) {
 
 hb_status launch_adjoint(Op* op, const double* q, const double* lam, double* q_bar,
                          double* c_bar, const double* coeff, double* work, cudaStream_t s) {
-  if (op->adjfrag) return launch_adjoint_f64(op, q, lam, q_bar, c_bar, coeff, work, s);
+  if (adjoint_f64_ready(op, s))
+    return launch_adjoint_f64(op, q, lam, q_bar, c_bar, coeff, work, s);
   const int dim = op->d->dim;
   switch (op->model) {
     case HB_MODEL_ADVECTION:

@@ -25,11 +25,27 @@ static hb_status adj_dispatch(const AdjCall& c) {
   }
 }
 
-hb_status prepare_adjoint_f64(Op* op) {
-  AdjCall c = {};
-  c.op = op;
-  c.configure = true;
-  return adj_dispatch(c);
+bool adjoint_f64_ready(Op* op, cudaStream_t s) {
+  const int state = op->adj_state.load(std::memory_order_acquire);
+  if (state) return state == 1;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (op->d->order > 7 || cudaStreamIsCapturing(s, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  std::lock_guard<std::mutex> lock(op->adj_mutex);
+  if (op->adj_state.load(std::memory_order_acquire) == 0) {
+    // (allocating here must not upset a capture on another thread)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    AdjCall c = {};
+    c.op = op;
+    c.configure = true;
+    op->adj_state.store(adj_dispatch(c) == HB_OK ? 1 : 2, std::memory_order_release);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  return op->adj_state.load(std::memory_order_acquire) == 1;
 }
 
 hb_status launch_adjoint_f64(Op* op, const double* q, const double* lam, double* q_bar,

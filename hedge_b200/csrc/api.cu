@@ -323,10 +323,6 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
     st = op->precision == HB_PREC_FP64 ? prepare_f64(op) : HB_ERR_UNSUPPORTED;
     if (st == HB_ERR_UNSUPPORTED) st = prepare_simt(op);
   }
-  if (!st && model != HB_MODEL_VARADV && d->order <= 7) {
-    st = prepare_adjoint_f64(op);
-    if (st == HB_ERR_UNSUPPORTED) st = HB_OK;   // the CUDA-core adjoint
-  }
   if (st) return bail(st);
   *out = reinterpret_cast<hb_op*>(op);
   return HB_OK;
@@ -533,11 +529,12 @@ hb_status hb_adjoint_stage(hb_op* handle, double a, double b, double dt, const d
     return fail(HB_ERR_INVALID_ARGUMENT, "adjoint stage: aliasing vectors");
   const hb_status st = check_adjoint(op, q, c_bar, coeff);
   if (st) return st;
-  if (!op->adjfrag)
-    return fail(HB_ERR_UNSUPPORTED, "adjoint stage: orders 1 to 7 (compose it from "
-                                    "hb_rhs_adjoint)");
   DeviceGuard g(op->d->device);
   if (!g.ok) return fail(HB_ERR_CUDA, "cannot select the CUDA device");
+  if (!adjoint_f64_ready(op, reinterpret_cast<cudaStream_t>(stream)))
+    return fail(HB_ERR_UNSUPPORTED, "adjoint stage: orders 1 to 7, and not as an operator's first "
+                                    "adjoint under stream capture (compose it from "
+                                    "hb_rhs_adjoint)");
   return launch_adjoint_stage(op, a, b, dt, q, lam, lq, c_bar, coeff, static_cast<double*>(work),
                               reinterpret_cast<cudaStream_t>(stream));
 }

@@ -753,23 +753,24 @@ class CompiledOperator:
             lam += b lq;  lq += dt (dR/dq)^T lam;  c_bar += dt (dR/dc)^T lam;
             lam *= a
 
-        (hb_adjoint_stage: two launches; beyond order 7 composed from
-        ``adjoint``)."""
-        if self.discr.order > 7:
-            lam.add_(lq, alpha=b)
-            q_bar, cb = self.adjoint(lam, q=q, coeff=coeff, want_c=c_bar is not None)
-            lq.add_(q_bar, alpha=dt)
-            if c_bar is not None:
-                c_bar.add_(cb, alpha=dt)
-            lam.mul_(a)
-            return
+        (hb_adjoint_stage: two launches; where that refuses, beyond order 7,
+        composed from ``adjoint``)."""
         c = self._coeff if coeff is None else coeff
-        _native.check(self._lib.hb_adjoint_stage(
+        st = self._lib.hb_adjoint_stage(
             self._handle, float(a), float(b), float(dt),
             q.data_ptr() if q is not None else None, lam.data_ptr(), lq.data_ptr(),
             c_bar.data_ptr() if c_bar is not None else None,
             c.data_ptr() if c is not None else None, self._adjoint_work().data_ptr(),
-            self._stream()))
+            self._stream())
+        if st != _native.HB_ERR_UNSUPPORTED:
+            _native.check(st)
+            return
+        lam.add_(lq, alpha=b)
+        q_bar, cb = self.adjoint(lam, q=q, coeff=coeff, want_c=c_bar is not None)
+        lq.add_(q_bar, alpha=dt)
+        if c_bar is not None:
+            c_bar.add_(cb, alpha=dt)
+        lam.mul_(a)
 
     def check(self):
         """Synchronise and raise if a kernel flagged bad input."""
