@@ -313,8 +313,11 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
   } else if (op->precision == HB_PREC_FP32 && desc->precision != HB_PREC_FP32_SIMT) {
     // FP32 state on the tensor cores where a resident kernel is built for
     // this (model, dimension, order), else on the CUDA cores
-    st = prepare_split(op);
-    op->split = st == HB_OK;
+    st = prepare_f64(op);
+    if (st == HB_ERR_UNSUPPORTED) {
+      st = prepare_split(op);
+      op->split = st == HB_OK;
+    }
     if (st == HB_ERR_UNSUPPORTED) {
       free_split(op);
       st = prepare_simt(op);

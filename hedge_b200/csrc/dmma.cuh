@@ -60,6 +60,16 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* g) {
                "l"(g)
                : "memory");
 }
+template <typename T>
+__device__ __forceinline__ void cp_async_word(T* smem, const T* g) {
+  if constexpr (sizeof(T) == 8)
+    cp_async8(smem, g);
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(smem)),
+                 "l"(g)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
 }

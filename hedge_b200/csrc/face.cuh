@@ -27,8 +27,8 @@ struct FaceExt {
 
 // Requests the exterior values of face node k; `nbr_node` maps (perm,
 // neighbour's face, k) to the neighbour's volume node.
-template <int MODEL, int DIM, bool VM>
-__device__ __forceinline__ void face_load(const FaceArgs<double>& a, const int2 cn, int k,
+template <int MODEL, int DIM, bool VM, typename S>
+__device__ __forceinline__ void face_load(const FaceArgs<S>& a, const int2 cn, int k,
                                           int64_t Knp, int np, int nfp, int nf, int nperm,
                                           const uint8_t* nbr_node,
                                           FaceExt<MODEL, DIM, double>& x) {
@@ -47,7 +47,7 @@ __device__ __forceinline__ void face_load(const FaceArgs<double>& a, const int2 
     const int64_t hi = h * nfp + k;
     if constexpr (C != 0) x.u[0] = a.halo_c[hi];
 #pragma unroll
-    for (int f = 0; f < F; ++f) x.u[C + f] = a.halo[hi * F + f];
+    for (int f = 0; f < F; ++f) x.u[C + f] = (double)a.halo[hi * F + f];
     return;
   }
   const int nface = cn.y & 3, perm = cn.y >> 2;
@@ -59,7 +59,7 @@ __device__ __forceinline__ void face_load(const FaceArgs<double>& a, const int2 
   const int64_t gi = (int64_t)cn.x * np + nbr_node[(perm * nf + nface) * nfp + k];
   if constexpr (C != 0) x.u[0] = __ldg(a.coeff + gi);
 #pragma unroll
-  for (int f = 0; f < F; ++f) x.u[C + f] = __ldg(a.q + f * Knp + gi);
+  for (int f = 0; f < F; ++f) x.u[C + f] = (double)__ldg(a.q + f * Knp + gi);
   if constexpr (VM) {
     x.eps = __ldg(a.coeff + gi);
     x.mu = __ldg(a.coeff + Knp + gi);
@@ -68,8 +68,8 @@ __device__ __forceinline__ void face_load(const FaceArgs<double>& a, const int2 
 
 // Flux of the interior values uM and the loaded exterior; own: this side's
 // volume node.  False: the face carries no flux.
-template <int MODEL, int DIM, bool VM>
-__device__ __forceinline__ bool face_flux(const FaceArgs<double>& a, const ModelParams& mp,
+template <int MODEL, int DIM, bool VM, typename S>
+__device__ __forceinline__ bool face_flux(const FaceArgs<S>& a, const ModelParams& mp,
                                           const int2 cn, int k, int nfp, int64_t own,
                                           int64_t Knp,
                                           const double (&uM)[Args<MODEL, DIM>::N],

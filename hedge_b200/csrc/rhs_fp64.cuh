@@ -54,7 +54,9 @@ namespace hb {
 
 __host__ __device__ constexpr int f64_ru8(int x) { return (x + 7) / 8 * 8; }
 
-template <int MODEL, int DIM, int ORDER>
+// SB: bytes of a state value (8: FP64, 4: FP32 state and residual; the
+// arithmetic is FP64 either way)
+template <int MODEL, int DIM, int ORDER, int SB = 8>
 struct F64Shape {
   static constexpr int F = Traits<MODEL, DIM>::F;
   static constexpr int C = Traits<MODEL, DIM>::COEFF;
@@ -103,7 +105,7 @@ struct F64Shape {
       COLS * LDZ > KG * COLS * LDP ? COLS * LDZ : KG * COLS * LDP;
   static constexpr size_t oZ = 0;
   static constexpr size_t oQ = al(oZ + 8 * zdoubles);          // [F][EB][NP]
-  static constexpr size_t oC = al(oQ + 8 * F * ENP);           // [2][EB][NP]
+  static constexpr size_t oC = al(oQ + SB * F * ENP);          // [2][EB][NP]
   static constexpr size_t oG = al(oC + 2 * 8 * C * ENP);       // [EB][G]
   static constexpr size_t oN = al(oG + 8 * EB * G);            // [EB][NF] int2
   static constexpr size_t oFm = al(oN + 8 * EB * NF);          // uint8 face nodes
@@ -119,17 +121,18 @@ struct F64Shape {
   }
 };
 
+template <typename IO>
 struct F64Args {
   int64_t K, nbatch, e_begin, e_end;
   int E, nperm;
-  FaceArgs<double> face;     // neighbour, halo and boundary sources
+  FaceArgs<IO> face;         // neighbour, halo and boundary sources
   const double2* afrag;      // operator fragments [STEPS][MT][32]
   const double* geo;
   const int2* conn;
   const int* fmask;
   const int* shuffle;
-  double* q_out;
-  double* res;
+  IO* q_out;
+  IO* res;
   const double* source;
   double ra, rb, dt;
   int mode;                  // 0: write rhs, 1: LSRK stage
@@ -137,11 +140,11 @@ struct F64Args {
 };
 
 // VM: Maxwell with variable material (coeff = [eps | mu])
-template <int MODEL, int DIM, int ORDER, bool VM>
-__global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
-                                  (F64Shape<MODEL, DIM, ORDER>::min_ctas(VM)))
-    rhs_fp64_kernel(const F64Args a) {
-  using S = F64Shape<MODEL, DIM, ORDER>;
+template <int MODEL, int DIM, int ORDER, bool VM, typename IO>
+__global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER, sizeof(IO)>::THREADS,
+                                  (F64Shape<MODEL, DIM, ORDER, sizeof(IO)>::min_ctas(VM)))
+    rhs_fp64_kernel(const F64Args<IO> a) {
+  using S = F64Shape<MODEL, DIM, ORDER, sizeof(IO)>;
   constexpr int F = S::F, C = S::C, NP = S::NP, NFP = S::NFP, NF = S::NF, NFPT = S::NFPT;
   constexpr int G = S::G, LDZ = S::LDZ, ENP = S::ENP, THREADS = S::THREADS;
   constexpr int MT = S::MT, RN = S::RN, KG = S::KG;
@@ -169,11 +172,11 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
   auto fetch = [&](int64_t batch, int buf) {
     const int64_t el0 = a.e_begin + batch * a.E;
     const int ne = (int)(a.e_end - el0 < a.E ? a.e_end - el0 : a.E);
-    double* dq = reinterpret_cast<double*>(smem + S::oQ);
+    IO* dq = reinterpret_cast<IO*>(smem + S::oQ);
     for (int x = tid; x < ne * NP; x += THREADS) {
 #pragma unroll
       for (int f = 0; f < F; ++f)
-        cp_async8(dq + f * ENP + x, a.face.q + f * Knp + el0 * NP + x);
+        cp_async_word(dq + f * ENP + x, a.face.q + f * Knp + el0 * NP + x);
       if constexpr (C != 0)
         cp_async8(reinterpret_cast<double*>(smem + S::oC) + buf * ENP + x,
                   a.face.coeff + el0 * NP + x);
@@ -185,7 +188,7 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
     cp_async_commit();
   };
 
-  const double* sq = reinterpret_cast<const double*>(smem + S::oQ);
+  const IO* sq = reinterpret_cast<const IO*>(smem + S::oQ);
   const double* sgeo = reinterpret_cast<const double*>(smem + S::oG);
   const int2* sconn = reinterpret_cast<const int2*>(smem + S::oN);
   if (blockIdx.x < a.nbatch) fetch(blockIdx.x, 0);
@@ -198,10 +201,10 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
     __syncthreads();   // the batch has arrived; the previous one is done with Z
 
     if (a.mode != 0) {
-      constexpr int LINES = (ENP * 8 + 127) / 128 + 1;
+      constexpr int LINE = 128 / sizeof(IO), LINES = (ENP + LINE - 1) / LINE + 1;
       for (int x = tid; x < F * LINES; x += THREADS) {
-        const int f = x / LINES, o = (x - f * LINES) * 16;
-        const double* r = a.res + f * Knp + el0 * NP + (o < ne * NP ? o : ne * NP - 1);
+        const int f = x / LINES, o = (x - f * LINES) * LINE;
+        const IO* r = a.res + f * Knp + el0 * NP + (o < ne * NP ? o : ne * NP - 1);
         asm volatile("prefetch.global.L2 [%0];" ::"l"(r));
       }
     }
@@ -222,7 +225,7 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
       const int e = x / NP, j = x - e * NP;
       double q[F];
 #pragma unroll
-      for (int f = 0; f < F; ++f) q[f] = sq[f * ENP + x];
+      for (int f = 0; f < F; ++f) q[f] = (double)sq[f * ENP + x];
       const double* ge = sgeo + e * G;
       double* z = sZ + e * F * LDZ + j;
 #pragma unroll
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
       double uM[F + C], n[DIM], fl[F];
       if constexpr (C != 0) uM[0] = sc[e * NP + lnode];
 #pragma unroll
-      for (int f = 0; f < F; ++f) uM[C + f] = sq[f * ENP + e * NP + lnode];
+      for (int f = 0; f < F; ++f) uM[C + f] = (double)sq[f * ENP + e * NP + lnode];
       const double* gf = sgeo + e * G + DIM * DIM + fc * (DIM + 1);
 #pragma unroll
       for (int d = 0; d < DIM; ++d) n[d] = gf[d];
@@ -329,7 +332,7 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
     // the state and residual at this thread's outputs, requested before the
     // barrier (from L2: the state's shared copy is being refilled, the
     // residual was prefetched)
-    double rv[S::UR][F], qv[S::UR][F];
+    IO rv[S::UR][F], qv[S::UR][F];
     const int64_t base = el0 * NP + tid;
     if (a.mode != 0) {
 #pragma unroll
@@ -373,11 +376,11 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
         }
         const int64_t gi = f * Knp + node;
         if (a.mode == 0) {
-          a.q_out[gi] = r;
+          a.q_out[gi] = (IO)r;
         } else {
-          const double nr = a.ra * rv[u][f] + a.dt * r;
-          a.res[gi] = nr;
-          a.q_out[gi] = qv[u][f] + a.rb * nr;
+          const double nr = a.ra * (double)rv[u][f] + a.dt * r;
+          a.res[gi] = (IO)nr;
+          a.q_out[gi] = (IO)((double)qv[u][f] + a.rb * nr);
         }
       }
     }
@@ -400,12 +403,12 @@ struct F64Call {
   bool configure;
 };
 
-template <int MODEL, int DIM, int ORDER, bool VM>
+template <int MODEL, int DIM, int ORDER, bool VM, typename IO>
 hb_status f64_one(const F64Call& c) {
-  using S = F64Shape<MODEL, DIM, ORDER>;
+  using S = F64Shape<MODEL, DIM, ORDER, sizeof(IO)>;
   Op* op = c.op;
   Discr* d = op->d;
-  auto kern = rhs_fp64_kernel<MODEL, DIM, ORDER, VM>;
+  auto kern = rhs_fp64_kernel<MODEL, DIM, ORDER, VM, IO>;
   if (c.configure) {
     if (d->np != S::NP || d->nfp != S::NFP)
       return fail(HB_ERR_UNSUPPORTED, "element sizes do not match the order");
@@ -447,7 +450,7 @@ hb_status f64_one(const F64Call& c) {
       return fail(HB_ERR_CUDA, "cannot upload the FP64 operator fragments");
     return HB_OK;
   }
-  F64Args a;
+  F64Args<IO> a;
   a.K = d->K;
   a.e_begin = c.e0;
   a.e_end = c.e1;
@@ -456,11 +459,11 @@ hb_status f64_one(const F64Call& c) {
   a.nbatch = (c.e1 - c.e0 + a.E - 1) / a.E;
   a.nperm = d->nperm;
   a.face.K = d->K;
-  a.face.q = static_cast<const double*>(c.q_in);
+  a.face.q = static_cast<const IO*>(c.q_in);
   a.face.coeff = c.coeff;
   a.face.bdry = c.bdry;
   a.face.n_given = op->n_given;
-  a.face.halo = static_cast<const double*>(op->halo);
+  a.face.halo = static_cast<const IO*>(op->halo);
   a.face.halo_c = op->halo_c;
   a.face.n_halo = op->n_halo;
   a.face.err = op->err_flag;
@@ -469,8 +472,8 @@ hb_status f64_one(const F64Call& c) {
   a.conn = op->conn;
   a.fmask = d->fmask;
   a.shuffle = d->shuffle;
-  a.q_out = static_cast<double*>(c.q_out);
-  a.res = static_cast<double*>(c.res);
+  a.q_out = static_cast<IO*>(c.q_out);
+  a.res = static_cast<IO*>(c.res);
   a.source = c.source;
   a.ra = c.ra;
   a.rb = c.rb;
@@ -491,27 +494,60 @@ hb_status f64_one(const F64Call& c) {
   return HB_OK;
 }
 
-constexpr int F64_MAX_ORDER = 7;
+// FP32 states that run here, in FP64 arithmetic, instead of on the split FP16
+// planes (or, where no such instance is built, on the CUDA cores): the smaller
+// elements, whose planes are mostly padding and whose batches are too short for
+// the split kernel's pipeline.  LSRK4 step, split or CUDA cores -> here: 3D
+// Maxwell N = 3, K = 48000 709 -> 608 us, K = 1296 58 -> 39 us; 3D wave N = 3,
+// K = 48000 417 -> 395 us; 2D wave N = 3, K = 45000 225 -> 97 us, N = 6, K = 20000
+// 140 -> 137 us; against 3D Maxwell N = 4, K = 48000 716 -> 1152 us and 3D wave
+// N = 4 489 -> 722 us, N = 5, K = 16464 252 -> 568 us.
+// On meshes beyond 16384 elements not 2D advection and wave of order 6 (wave, K =
+// 33800: 201 -> 210 us) and 3D wave of order 1 and 2 (K = 34992: 63 -> 67 and
+// 143 -> 146 us); on smaller ones those too (K = 7200 81 -> 72, K = 10368 52 -> 32 us).
+constexpr bool f64_fp32_state(int model, int dim, int order) {
+  (void)model;
+  return dim == 2 || order <= 3;
+}
+inline bool f64_fp32_mesh(int model, int dim, int order, int64_t k) {
+  const bool wave = model == HB_MODEL_WAVE || model == HB_MODEL_VARWAVE;
+  const bool even = dim == 2 ? order == 6 && (wave || model == HB_MODEL_ADVECTION)
+                             : order <= 2 && wave;
+  return !even || k <= 16384;
+}
+
+template <int MODEL, int DIM, int ORDER>
+hb_status f64_order(const F64Call& c) {
+  if (c.op->precision == HB_PREC_FP32) {
+    // FP32 states: the elements and meshes that are faster here; no variable
+    // material
+    if constexpr (f64_fp32_state(MODEL, DIM, ORDER)) {
+      if (!c.configure || f64_fp32_mesh(MODEL, DIM, ORDER, c.op->d->K))
+        return f64_one<MODEL, DIM, ORDER, false, float>(c);
+    }
+    return fail(HB_ERR_UNSUPPORTED, "FP64 tensor-core kernel: not for this FP32 state");
+  }
+  if constexpr (IsMaxwell<MODEL>::value) {
+    if (c.configure || c.coeff != nullptr) {
+      const hb_status st = f64_one<MODEL, DIM, ORDER, true, double>(c);
+      if (st || !c.configure) return st;
+    }
+  }
+  return f64_one<MODEL, DIM, ORDER, false, double>(c);
+}
 
 template <int MODEL, int DIM>
 hb_status f64_orders(const F64Call& c) {
-  const bool vm = IsMaxwell<MODEL>::value && c.coeff != nullptr;
   switch (c.op->d->order) {
-#define HB_CASE(O)                                                         \
-  case O:                                                                  \
-    if constexpr (IsMaxwell<MODEL>::value) {                               \
-      if (c.configure) {                                                   \
-        const hb_status st = f64_one<MODEL, DIM, O, true>(c);              \
-        if (st) return st;                                                 \
-      }                                                                    \
-      if (vm) return f64_one<MODEL, DIM, O, true>(c);                      \
-    }                                                                      \
-    return f64_one<MODEL, DIM, O, false>(c);
-    HB_CASE(1) HB_CASE(2) HB_CASE(3) HB_CASE(4) HB_CASE(5) HB_CASE(6) HB_CASE(7)
-#undef HB_CASE
+    case 1: return f64_order<MODEL, DIM, 1>(c);
+    case 2: return f64_order<MODEL, DIM, 2>(c);
+    case 3: return f64_order<MODEL, DIM, 3>(c);
+    case 4: return f64_order<MODEL, DIM, 4>(c);
+    case 5: return f64_order<MODEL, DIM, 5>(c);
+    case 6: return f64_order<MODEL, DIM, 6>(c);
+    case 7: return f64_order<MODEL, DIM, 7>(c);
     default: return fail(HB_ERR_UNSUPPORTED, "FP64 tensor-core kernel: orders 1 to 7");
   }
-  (void)vm;
 }
 
 }  // namespace hb
