@@ -33,6 +33,7 @@ constexpr int ENS_MAX_F = 4;   // wave in 3D
 
 struct EnsInst {
   int model, F, dim, np, nfp, nperm, G;
+  int order;              // 1 to 7 where np and nfp are that order's, else 0
   int64_t K;
   const float* dmats_t;   // [dim][np(j)][np(i)]
   const float* lift_t;    // [nfpt][np]
@@ -45,6 +46,14 @@ struct EnsInst {
   double dt;
   ModelParams mp;
 };
+
+// the order whose element sizes a discretization has, 0 if none of 1 to 7
+inline int ens_order(const Discr* d) {
+  const int o = d->order;
+  const int np = d->dim == 2 ? (o + 1) * (o + 2) / 2 : (o + 1) * (o + 2) * (o + 3) / 6;
+  const int nfp = d->dim == 2 ? o + 1 : (o + 1) * (o + 2) / 2;
+  return o >= 1 && o <= 7 && d->np == np && d->nfp == nfp ? o : 0;
+}
 
 struct EnsTile {
   int inst, E;
@@ -81,13 +90,20 @@ __host__ __device__ inline EnsLayout ens_layout(const EnsSizes& z) {
   return L;
 }
 
-template <int MODEL, int DIM>
-__device__ void ens_tile(const EnsInst& I, const EnsTile& T, const EnsLayout& L,
+// ORDER: 1 to 7, compile-time loop bounds and divisors; 0: any order
+template <int MODEL, int DIM, int ORDER>
+__device__ __forceinline__ void ens_tile(const EnsInst& I, const EnsTile& T, const EnsLayout& L,
                          unsigned char* smem, double ra, double rb, int src, int* err) {
   constexpr int F = Traits<MODEL, DIM>::F;
   constexpr int NA = F;   // no coefficient field in the batch models
   constexpr int NF = DIM + 1;
-  const int np = I.np, nfp = I.nfp, G = I.G, E = T.E, ne = T.ne;
+  constexpr int UNROLL = ORDER ? 4 : 1;
+  constexpr int CNP = DIM == 2 ? (ORDER + 1) * (ORDER + 2) / 2
+                               : (ORDER + 1) * (ORDER + 2) * (ORDER + 3) / 6;
+  constexpr int CNFP = DIM == 2 ? ORDER + 1 : (ORDER + 1) * (ORDER + 2) / 2;
+  const int np = ORDER ? CNP : I.np, nfp = ORDER ? CNFP : I.nfp;
+  constexpr int G = DIM * DIM + NF * (DIM + 1);
+  const int E = T.E, ne = T.ne;
   const int nfpt = NF * nfp;
   const float* sD = reinterpret_cast<const float*>(smem + L.oD);
   const float* sL = reinterpret_cast<const float*>(smem + L.oL);
@@ -120,6 +136,7 @@ __device__ void ens_tile(const EnsInst& I, const EnsTile& T, const EnsLayout& L,
 #pragma unroll
       for (int f = 0; f < F; ++f) dr[r][f] = 0.f;
     const float* qe = sq + e * np;
+#pragma unroll UNROLL
     for (int j = 0; j < np; ++j) {
       float d[DIM];
 #pragma unroll
@@ -187,8 +204,13 @@ __device__ void ens_tile(const EnsInst& I, const EnsTile& T, const EnsLayout& L,
   for (int s = tid; s < ne * np; s += ENS_THREADS) {
     const int e = s / np, i = s - e * np;
     float acc[F];
+    double r0[F];   // the residual, requested ahead of the lift
 #pragma unroll
-    for (int f = 0; f < F; ++f) acc[f] = 0.f;
+    for (int f = 0; f < F; ++f) {
+      acc[f] = 0.f;
+      r0[f] = I.res[f * Knp + el0 * np + s];
+    }
+#pragma unroll UNROLL
     for (int p = 0; p < nfpt; ++p) {
       const float l = sL[p * np + i];
 #pragma unroll
@@ -199,21 +221,24 @@ __device__ void ens_tile(const EnsInst& I, const EnsTile& T, const EnsLayout& L,
       const double r = (double)model_finish<MODEL, DIM, float>(I.mp, f, sv[f * E * np + s],
                                                                 acc[f], 0.f);
       const int64_t idx = f * Knp + el0 * np + s;
-      const double nr = ra * I.res[idx] + I.dt * r;
+      const double nr = ra * r0[f] + I.dt * r;
       I.res[idx] = nr;
       q_out[idx] = (float)((double)sq[f * E * np + s] + rb * nr);
     }
   }
 }
 
-// 6 CTAs per SM (40 registers): the stage is latency-bound on its
-// global loads, and the extra resident warps hide more of that latency
-// than the few spilled registers cost (64 registers, 4 CTAs: 6.43 ms per
-// C5 step; 6 CTAs: 5.86 ms)
-__global__ void __launch_bounds__(ENS_THREADS, 6) ens_kernel(const EnsInst* __restrict__ insts,
-                                                           const EnsTile* __restrict__ tiles,
-                                                           int ntiles, EnsLayout L, double ra,
-                                                           double rb, int src, int* err) {
+// The stage waits on its global loads, and more resident warps hide more of
+// that than the spilled registers cost: in 2D 8 CTAs per SM (32 registers); in
+// 3D, whose nodes hold more values, 6 (40 registers).  Measured on 20 2D members
+// of order 3 to 6, K = 500 to 20000, per LSRK4 step: 560 us with run-time
+// element sizes at 6 CTAs; compile-time sizes 482 us; the residual requested
+// ahead of the lift 465 us; 8 CTAs 451 us.
+template <int DIM>
+__global__ void __launch_bounds__(ENS_THREADS, DIM == 2 ? 8 : 6) ens_kernel(const EnsInst* __restrict__ insts,
+                                                             const EnsTile* __restrict__ tiles,
+                                                             int ntiles, EnsLayout L, double ra,
+                                                             double rb, int src, int* err) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x;
   const float* cached = nullptr;   // operators resident in shared memory
@@ -233,17 +258,24 @@ __global__ void __launch_bounds__(ENS_THREADS, 6) ens_kernel(const EnsInst* __re
       for (int x = tid; x < I.nperm * I.nfp; x += ENS_THREADS) wsh[x] = I.shuffle[x];
       cached = I.dmats_t;
     }
-    if (I.dim == 2) {
-      if (I.model == HB_MODEL_ADVECTION)
-        ens_tile<HB_MODEL_ADVECTION, 2>(I, T, L, smem, ra, rb, src, err);
-      else
-        ens_tile<HB_MODEL_WAVE, 2>(I, T, L, smem, ra, rb, src, err);
-    } else {
-      if (I.model == HB_MODEL_ADVECTION)
-        ens_tile<HB_MODEL_ADVECTION, 3>(I, T, L, smem, ra, rb, src, err);
-      else
-        ens_tile<HB_MODEL_WAVE, 3>(I, T, L, smem, ra, rb, src, err);
+    const bool adv = I.model == HB_MODEL_ADVECTION;
+#define HB_ENS_ORDER(O)                                                                  \
+  case O:                                                                                \
+    if (adv)                                                                             \
+      ens_tile<HB_MODEL_ADVECTION, DIM, O>(I, T, L, smem, ra, rb, src, err);             \
+    else                                                                                 \
+      ens_tile<HB_MODEL_WAVE, DIM, O>(I, T, L, smem, ra, rb, src, err);                  \
+    break;
+    switch (I.order) {
+      HB_ENS_ORDER(1) HB_ENS_ORDER(2) HB_ENS_ORDER(3) HB_ENS_ORDER(4)
+      HB_ENS_ORDER(5) HB_ENS_ORDER(6) HB_ENS_ORDER(7)
+      default:
+        if (adv)
+          ens_tile<HB_MODEL_ADVECTION, DIM, 0>(I, T, L, smem, ra, rb, src, err);
+        else
+          ens_tile<HB_MODEL_WAVE, DIM, 0>(I, T, L, smem, ra, rb, src, err);
     }
+#undef HB_ENS_ORDER
   }
 }
 
@@ -254,7 +286,7 @@ struct Batch {
   EnsInst* d_insts = nullptr;
   EnsTile* d_tiles = nullptr;
   int* err = nullptr;
-  int ntiles = 0, grid = 0;
+  int ntiles = 0, grid = 0, dim = 2;
   EnsLayout L{};
   int64_t dofs = 0;
 };
@@ -289,6 +321,7 @@ hb_status batch_create(const hb_batch_member* m, int32_t n, Batch** out) {
     I.F = op->F;
     I.dim = d->dim;
     I.np = d->np;
+    I.order = ens_order(d);
     I.nfp = d->nfp;
     I.nperm = d->nperm;
     I.G = d->G;
@@ -345,10 +378,12 @@ hb_status batch_create(const hb_batch_member* m, int32_t n, Batch** out) {
           cudaSuccess)
     return bail(fail(HB_ERR_CUDA, "batch: device query"));
   if (B->L.total > (size_t)max_optin) return bail(fail(HB_ERR_UNSUPPORTED, "batch: tiles too large"));
-  if (cudaFuncSetAttribute(ens_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  auto kern = dim == 2 ? ens_kernel<2> : ens_kernel<3>;
+  B->dim = dim;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)B->L.total) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ens_kernel, ENS_THREADS,
-                                                    B->L.total) != cudaSuccess)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ENS_THREADS, B->L.total) !=
+          cudaSuccess)
     return bail(fail(HB_ERR_CUDA, "batch: occupancy query"));
   B->grid = std::max(1, std::min(B->ntiles, sms * std::max(per_sm, 1)));
   if (cudaMalloc(&B->d_insts, sizeof(EnsInst) * n) != cudaSuccess ||
@@ -376,8 +411,9 @@ void batch_destroy(Batch* B) {
 hb_status batch_stage(Batch* B, double a, double b, int parity, cudaStream_t s) {
   DeviceGuard g(B->device);
   if (!g.ok) return fail(HB_ERR_CUDA, "cannot select the CUDA device");
-  ens_kernel<<<B->grid, ENS_THREADS, B->L.total, s>>>(B->d_insts, B->d_tiles, B->ntiles, B->L,
-                                                      a, b, parity & 1, B->err);
+  auto kern = B->dim == 2 ? ens_kernel<2> : ens_kernel<3>;
+  kern<<<B->grid, ENS_THREADS, B->L.total, s>>>(B->d_insts, B->d_tiles, B->ntiles, B->L, a, b,
+                                                parity & 1, B->err);
   HB_CUDA(cudaGetLastError());
   return HB_OK;
 }
