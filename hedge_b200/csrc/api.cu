@@ -355,10 +355,15 @@ static hb_status check_inputs(Op* op, const void* q_in, const void* q_out,
     return fail(HB_ERR_INVALID_ARGUMENT, "variable-coefficient advection needs the velocity");
   const bool maxwell = op->model == HB_MODEL_MAXWELL || op->model == HB_MODEL_MAXWELL_TM ||
                        op->model == HB_MODEL_MAXWELL_TE;
-  if (maxwell && coeff && op->split)
+  // FP32 (HB_PREC_FP32) Maxwell of order 3 runs on rhs_fp64.cu's kernel, which
+  // could take both, but the precision's contract from order 3 on is the split
+  // kernels'
+  const bool fixed = op->split || (op->model == HB_MODEL_MAXWELL && op->afrag &&
+                                   op->precision == HB_PREC_FP32 && op->d->order >= 3);
+  if (maxwell && coeff && fixed)
     return fail(HB_ERR_UNSUPPORTED, "Maxwell with variable material: CUDA-core kernels only "
                                     "(HB_PREC_FP64, HB_PREC_FP32_SIMT)");
-  if (maxwell && bdry && op->split)
+  if (maxwell && bdry && fixed)
     return fail(HB_ERR_UNSUPPORTED, "Maxwell incident data: CUDA-core kernels only "
                                     "(HB_PREC_FP64, HB_PREC_FP32_SIMT)");
   return HB_OK;

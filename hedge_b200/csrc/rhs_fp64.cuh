@@ -516,24 +516,29 @@ inline bool f64_fp32_mesh(int model, int dim, int order, int64_t k) {
   return !even || k <= 16384;
 }
 
-template <int MODEL, int DIM, int ORDER>
-hb_status f64_order(const F64Call& c) {
-  if (c.op->precision == HB_PREC_FP32) {
-    // FP32 states: the elements and meshes that are faster here; no variable
-    // material
-    if constexpr (f64_fp32_state(MODEL, DIM, ORDER)) {
-      if (!c.configure || f64_fp32_mesh(MODEL, DIM, ORDER, c.op->d->K))
-        return f64_one<MODEL, DIM, ORDER, false, float>(c);
-    }
-    return fail(HB_ERR_UNSUPPORTED, "FP64 tensor-core kernel: not for this FP32 state");
-  }
+// Maxwell: the variable-material kernel where the call gives the material
+template <int MODEL, int DIM, int ORDER, typename IO>
+hb_status f64_material(const F64Call& c) {
   if constexpr (IsMaxwell<MODEL>::value) {
     if (c.configure || c.coeff != nullptr) {
-      const hb_status st = f64_one<MODEL, DIM, ORDER, true, double>(c);
+      const hb_status st = f64_one<MODEL, DIM, ORDER, true, IO>(c);
       if (st || !c.configure) return st;
     }
   }
-  return f64_one<MODEL, DIM, ORDER, false, double>(c);
+  return f64_one<MODEL, DIM, ORDER, false, IO>(c);
+}
+
+template <int MODEL, int DIM, int ORDER>
+hb_status f64_order(const F64Call& c) {
+  if (c.op->precision == HB_PREC_FP32) {
+    // FP32 states: the elements and meshes that are faster here
+    if constexpr (f64_fp32_state(MODEL, DIM, ORDER)) {
+      if (!c.configure || f64_fp32_mesh(MODEL, DIM, ORDER, c.op->d->K))
+        return f64_material<MODEL, DIM, ORDER, float>(c);
+    }
+    return fail(HB_ERR_UNSUPPORTED, "FP64 tensor-core kernel: not for this FP32 state");
+  }
+  return f64_material<MODEL, DIM, ORDER, double>(c);
 }
 
 template <int MODEL, int DIM>

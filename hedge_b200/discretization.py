@@ -48,10 +48,12 @@ class Discretization:
     FP32, and so is the arithmetic), "fp32", "fp64", "bf16x3" (FP64 state,
     differentiation and lift as split-BF16 tensor-core products with FP32
     accumulation) or "fp16x3" (the same with FP16 planes of power-of-two
-    scaled rows: same cost, ~8x smaller error).  "fp32" runs the two
-    contractions as FP16x3 tensor-core products where a resident tensor-core
-    kernel is built for the (model, dimension, order) and on CUDA cores
-    otherwise; "fp32-simt" keeps them on CUDA cores.
+    scaled rows: same cost, ~8x smaller error).  "fp32" keeps
+    the state in FP32: in 2D and up to order 3 in 3D the arithmetic is FP64
+    (FP64 tensor cores); beyond, and on some large meshes, the contractions
+    are FP16x3 tensor-core products where a resident kernel is built for the
+    (model, dimension, order), else FP32 on CUDA cores; "fp32-simt" keeps
+    FP32 arithmetic on CUDA cores.
     """
 
     def __init__(self, mesh: Mesh, order=None, local_discretization=None,
@@ -444,7 +446,8 @@ class CompiledOperator:
         prec = PRECISIONS[precision] if precision != "plain" else (
             _native.PREC_FP64 if discr.default_scalar_type == np.float64
             else _native.PREC_FP32)
-        # Maxwell with variable material or incident data: the CUDA-core kernels
+        # Maxwell with variable material or incident data: FP64, or FP32 on the
+        # CUDA cores
         self.var_material = bool(ot.params.get("variable_material"))
         self.incident_data = bool(ot.params.get("incident_data"))
         self.given_rows = ot.n_fields if self.incident_data else 1

@@ -404,7 +404,7 @@ class MaxwellOperator(HyperbolicOperator):
     variable material, volume fields: given functions
     (TimeConstantGivenFunction, ``volume_interpolant(t, discr)``), callables
     f(x) of the node coordinates, volume vectors [K*Np], or template fields.
-    Variable material runs on the CUDA-core kernels (fp64, fp32)."""
+    Variable material runs in fp64 (FP64 tensor cores) and fp32 (CUDA cores)."""
 
     _default_dimensions = 3
     model_id = MODEL_MAXWELL
@@ -424,7 +424,7 @@ class MaxwellOperator(HyperbolicOperator):
         (every kernel); incident data given per call as boundary vectors
         (template fields outside any BoundarizeOperator, one per carried
         component, e.g. ``make_sym_vector("inc", n_fields)``) runs on the
-        CUDA-core kernels."""
+        fp64 and fp32 CUDA-core kernels."""
         self.dimensions = dimensions or self._default_dimensions
         if self.dimensions != self._default_dimensions:
             raise NotImplementedError("%s is a %dD system" % (type(self).__name__,

@@ -50,10 +50,12 @@ enum {
 
 enum {
   HB_PREC_FP64 = 0,   /* FP64 state, FP64 arithmetic */
-  HB_PREC_FP32 = 1,   /* FP32 state and residual, FP32 arithmetic; where a resident
-                         tensor-core kernel is built for the (model, dimension,
-                         order), the two contractions run as split-FP16 products
-                         (as HB_PREC_FP16X3, FP32 accumulation), else on CUDA cores
+  HB_PREC_FP32 = 1,   /* FP32 state and residual.  In 2D and up to order 3 in 3D the
+                         arithmetic is FP64 (FP64 tensor cores); where a resident
+                         tensor-core kernel is built for the (model, dimension, order)
+                         beyond that (and, on large meshes, for the sizes it is faster
+                         at) the two contractions are FP16-split products of scaled rows
+                         (as HB_PREC_FP16X3, FP32 accumulation); else FP32 on CUDA cores
                          (hedge/discretization/__init__.py:217-219,
                          default_scalar_type float32) */
   HB_PREC_BF16X3 = 2, /* FP64 state, split-BF16 tensor-core products, FP32 accumulation */

@@ -85,3 +85,68 @@ def test_every_order(cuda_device, model, dim, order):
                                            ("varwave", 3, 16, 13)])
 def test_mesh_sizes(cuda_device, model, dim, n, m):
     _check(model, dim, 2, n, m)
+
+
+@pytest.mark.parametrize("order", range(1, 8))
+@pytest.mark.parametrize("model,dim", [m for m in MODELS if m[0] != "material"])
+def test_fp32_state(cuda_device, model, dim, order):
+    """FP32 states, on this kernel or (3D from order 4) on the split planes:
+    1e-5 relative L2, the FP32 path's bound, on FP32-rounded inputs."""
+    _check_fp32(model, dim, order, *((3, 5) if dim == 2 else (1, 2 if order > 5 else 5)))
+
+
+@pytest.mark.parametrize("n,m", [(90, 91), (91, 91)])
+def test_fp32_state_on_both_sides_of_the_mesh_rule(cuda_device, n, m):
+    """2D wave of order 6 with 16380 and 16562 elements: this kernel, the split
+    planes."""
+    _check_fp32("wave", 2, 6, n, m)
+
+
+def _check_fp32(model, dim, order, n, m):
+    from oracle import OracleRHS
+    d = hb.Discretization(_mesh(dim, n, m), order=order, precision="fp32")
+    op = _operator(model, dim, d)
+    comp = d.compile(op.op_template())
+    x = d.nodes
+    w = np.stack([np.sin((f + 1.3) * x[:, 0] + f) * np.cos(x[:, -1]) for f in range(comp.F)])
+    w = w.astype(np.float32).astype(np.float64)
+    bc = np.sin(3 * d.get_boundary("wall").nodes[:, 0]) if model == "advection" else None
+    ref = OracleRHS(d, op.descriptor())(w, bc_in=bc)
+    q = d.to_device(w)
+    out = q.new_empty(q.shape)
+    comp.rhs_into(q, out, bc_in=bc)
+    comp.check()
+    assert rel_l2(out.double().cpu().numpy(), ref) <= 1e-5
+
+
+@pytest.mark.parametrize("order", [2, 3])
+def test_fp32_material_and_incident_data(cuda_device, order):
+    """HB_PREC_FP32 Maxwell through the C ABI: variable material and incident
+    data are taken at order 2 and refused from order 3 on, where the precision
+    is the split kernels'."""
+    import ctypes as C
+
+    from hedge_b200 import _native
+    from hedge_b200.discretization import op_descriptor
+    from oracle import OracleRHS
+    d = hb.Discretization(_mesh(3, 1, 5), order=order, precision="fp32")
+    op = _operator("material", 3, d)
+    comp = d.compile(op.op_template())
+    desc = op_descriptor(comp.ot, _native.PREC_FP32, comp.conn, comp.n_given)
+    h = C.c_void_p()
+    _native.check(comp._lib.hb_op_create(d._native_handle(), C.byref(desc), C.byref(h)))
+    rng = np.random.default_rng(5)
+    w = rng.uniform(-1, 1, (6, len(d))).astype(np.float32).astype(np.float64)
+    q = d.to_device(w)
+    out = q.new_empty(q.shape)
+    st = comp._lib.hb_rhs(h, q.data_ptr(), out.data_ptr(), comp._coeff.data_ptr(), None, None,
+                          comp._stream())
+    if order == 3:
+        assert st == _native.HB_ERR_UNSUPPORTED
+        assert comp._lib.hb_rhs(h, q.data_ptr(), out.data_ptr(), None, q.data_ptr(), None,
+                                comp._stream()) == _native.HB_ERR_UNSUPPORTED
+    else:
+        _native.check(st)
+        ref = OracleRHS(d, op.descriptor())(w)
+        assert rel_l2(out.double().cpu().numpy(), ref) <= 1e-5
+    _native.check(comp._lib.hb_op_destroy(h))
