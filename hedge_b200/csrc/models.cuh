@@ -277,21 +277,21 @@ __device__ __forceinline__ void maxwell_flux3_var(const ModelParams& mp, bool bd
 #pragma unroll
     for (int k = 0; k < 3; ++k) f[3 + k] = T(0.5) * t[k];
   } else {
-    const T Yi = T(1) / Zi, Ye = T(1) / Ze;
+    // -1 / (Zi + Ze) n x (Ze [H] - alpha n x [E]) and, with Y = 1 / Z,
+    // 1 / (Yi + Ye) n x (Ye [E] + alpha n x [H]), over one division: 1 / (Yi + Ye) =
+    // Zi Ze / (Zi + Ze)
+    const T s = T(1) / (Zi + Ze), zi = Zi * s, zz = alpha * (zi * Ze);
     T nde[3], ndh[3], a[3];
     cross3(n, de, nde);
     cross3(n, dh, ndh);
 #pragma unroll
     for (int k = 0; k < 3; ++k) a[k] = Ze * dh[k] - alpha * nde[k];
     cross3(n, a, t);
-    const T fe = T(-1) / (Zi + Ze), fh = T(1) / (Yi + Ye);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) f[k] = fe * t[k];
+    for (int k = 0; k < 3; ++k) f[k] = -s * t[k];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) a[k] = Ye * de[k] + alpha * ndh[k];
-    cross3(n, a, t);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) f[3 + k] = fh * t[k];
+    for (int k = 0; k < 3; ++k) a[k] = zi * de[k] + zz * ndh[k];
+    cross3(n, a, &f[3]);
   }
 }
 

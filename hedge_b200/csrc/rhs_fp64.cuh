@@ -79,10 +79,12 @@ struct F64Shape {
   // few node tiles leave registers for more column tiles (and the batch then
   // has a node or a face point for every thread)
   static constexpr int RN = MT == 1 ? 8 : MT == 2 ? 4 : 2;
-  // two steps in flight where the tile and the model leave registers (stage
-  // times: 2D wave N = 3, K = 684 4.6 -> 4.3 us; Maxwell N = 2, K = 48000 58.6 ->
-  // 61.4 us, so not there)
-  static constexpr int UNROLL = MT <= 3 && F <= 3 ? 2 : 1;
+  // Two steps of the GEMM unrolled where the registers and the instruction
+  // cache bear it, by measurement (stage times, one -> two): 3D Maxwell N = 5,
+  // K = 13182 139 -> 123 us, N = 4, K = 48000 258 -> 240 us, 2D wave N = 3, K = 684
+  // 4.6 -> 4.3 us; but 3D Maxwell N = 2, K = 48000 58.6 -> 61.4 us, 2D TM N = 6, K =
+  // 33800 41.9 -> 44.7 us.
+  static constexpr int UNROLL = (DIM == 3 ? MT >= 4 || F <= 3 : MT <= 3) ? 2 : 1;
   static constexpr int NGW = 2;
   // from 11 node tiles a CTA fills the SM: four k shares give it 8 warps
   static constexpr int KG = MT >= 11 ? 4 : 2;
@@ -135,6 +137,7 @@ struct F64Args {
   IO* res;
   const double* source;
   double ra, rb, dt;
+  double inv_eps, inv_mu;    // fixed material
   int mode;                  // 0: write rhs, 1: LSRK stage
   ModelParams mp;
 };
@@ -348,7 +351,6 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER, sizeof(IO)>::THREA
     __syncthreads();
 
     // ---- output in linear order ----
-    const bool unit = !VM && a.mp.eps == 1.0 && a.mp.mu == 1.0;
 #pragma unroll
     for (int u = 0; u < S::UR; ++u) {
       const int n = tid + u * THREADS;
@@ -356,10 +358,11 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER, sizeof(IO)>::THREA
       const int e = n / NP, i = n - e * NP;
       const double* P = sZ + e * F * S::LDP + i;
       const int64_t node = base + u * THREADS;
-      double eps = a.mp.eps, mu = a.mp.mu;
+      double inv_eps = a.inv_eps, inv_mu = a.inv_mu;
       if constexpr (VM) {
-        eps = a.face.coeff[node];
-        mu = a.face.coeff[Knp + node];
+        // one division for the fields of a kind
+        inv_eps = 1.0 / a.face.coeff[node];
+        inv_mu = 1.0 / a.face.coeff[Knp + node];
       }
 #pragma unroll
       for (int f = 0; f < F; ++f) {
@@ -369,7 +372,7 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER, sizeof(IO)>::THREA
         const int64_t si = a.source ? model_src_index<MODEL>(f, node, Knp) : -1;
         const double src = si >= 0 ? a.source[si] : 0.0;
         if constexpr (IsMaxwell<MODEL>::value) {
-          if (!unit) r /= f < maxwell_ne<MODEL>() ? eps : mu;
+          r *= f < maxwell_ne<MODEL>() ? inv_eps : inv_mu;
           if (f < maxwell_ne<MODEL>()) r += src;
         } else {
           r = model_finish<MODEL, DIM, double>(a.mp, f, r, 0.0, src);
@@ -480,6 +483,8 @@ hb_status f64_one(const F64Call& c) {
   a.dt = c.dt;
   a.mode = c.mode;
   a.mp = op->mp;
+  a.inv_eps = 1.0 / op->mp.eps;
+  a.inv_mu = 1.0 / op->mp.mu;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)std::min<int64_t>(slots, a.nbatch));
   cfg.blockDim = dim3(S::THREADS);
