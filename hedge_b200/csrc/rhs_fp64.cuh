@@ -33,9 +33,9 @@
 // Bound: the FP64 pipe, which the MMAs share with the fluxes' FP64 arithmetic
 // (4 cycles per MMA and SM: 111 us of a C2 stage with the tile padding), and
 // beside it the latency of the point phases at 16 warps per SM.  Measured per
-// stage against the CUDA-core kernel: 3D Maxwell N = 4, K = 48000 454 -> 248
-// us, N = 5, K = 13182 333 -> 122 us, variable material N = 2, K = 12960 33 ->
-// 21 us; 3D wave N = 7, K = 10368 474 -> 234 us; 2D TM N = 5, K = 19594 33 ->
+// stage against the CUDA-core kernel: 3D Maxwell N = 4, K = 48000 454 -> 240
+// us, N = 5, K = 13182 333 -> 123 us, variable material N = 2, K = 12960 33 ->
+// 20 us; 3D wave N = 7, K = 10368 474 -> 239 us; 2D TM N = 5, K = 19594 33 ->
 // 18 us; 2D wave N = 3, K = 684 8.3 -> 4.2 us.  Reference
 // loops: jit/diff.py:137-175, jit/flux.py:311-353 and 429-472,
 // jit/lift.py:110-141, jit/__init__.py:501-519,
@@ -503,7 +503,7 @@ hb_status f64_one(const F64Call& c) {
 // planes (or, where no such instance is built, on the CUDA cores): the smaller
 // elements, whose planes are mostly padding and whose batches are too short for
 // the split kernel's pipeline.  LSRK4 step, split or CUDA cores -> here: 3D
-// Maxwell N = 3, K = 48000 709 -> 608 us, K = 1296 58 -> 39 us; 3D wave N = 3,
+// Maxwell N = 3, K = 9438 174 -> 141 us, K = 48000 709 -> 608 us, K = 1296 58 -> 39 us; 3D wave N = 3,
 // K = 48000 417 -> 395 us; 2D wave N = 3, K = 45000 225 -> 97 us, N = 6, K = 20000
 // 140 -> 137 us; against 3D Maxwell N = 4, K = 48000 716 -> 1152 us and 3D wave
 // N = 4 489 -> 722 us, N = 5, K = 16464 252 -> 568 us.
