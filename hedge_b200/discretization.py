@@ -23,8 +23,8 @@ from .facegroups import Boundary, build_compact_connectivity, build_interior_fac
 from .mesh import Mesh, TAG_ALL, TAG_NONE
 from .lowering import as_descriptor
 from .optemplate import Expr
-from .models import (BC_GIVEN, BC_INCIDENT, BC_NONE, MODEL_MAXWELL, MODEL_MAXWELL_TE,
-                     MODEL_MAXWELL_TM, MODEL_VARADV, MODEL_VARWAVE, MODEL_WAVE,
+from .models import (BC_GIVEN, BC_INCIDENT, BC_NONE, CONTEXT_DATA, MODEL_MAXWELL,
+                     MODEL_MAXWELL_TE, MODEL_MAXWELL_TM, MODEL_VARADV, MODEL_VARWAVE, MODEL_WAVE,
                      MODEL_ADVECTION, OpTemplate, TimeConstantGivenFunction)
 from .quadrature import ElementQuadrature
 from .refelem import make_element
@@ -887,16 +887,20 @@ class BoundRHS:
         return {}
 
     def constant_context(self):
-        """Whether ``context`` is the same at all times: the model has no
-        boundary data or velocity to evaluate, or gives them as
-        TimeConstantGivenFunctions."""
+        """Whether ``context`` is known to be the same at all times: there is
+        no boundary data or velocity to evaluate, or this class and the model
+        evaluate it in their own ``context`` (not an override) and all that
+        it reads are TimeConstantGivenFunctions."""
+        if getattr(self.context, "__func__", None) is not BoundRHS.context:
+            return False
         comp = self.compiled
         if not comp.n_given and comp.ot.model != MODEL_VARADV:
             return True
-        given = [getattr(self.model, n, None)
-                 for n in ("inflow_u", "dirichlet_bc_f", "advec_v", "bc_u_f")]
-        return all(x is None or isinstance(x, str) or type(x) is TimeConstantGivenFunction
-                   for x in given)
+        ctx = getattr(self.model, "context", None)
+        read = CONTEXT_DATA.get(getattr(ctx, "__func__", None))
+        return read is not None and all(
+            x is None or isinstance(x, str) or type(x) is TimeConstantGivenFunction
+            for x in (getattr(ctx.__self__, name) for name in read))
 
     def __call__(self, t, w, **extra_context):
         kw = self.context(t)

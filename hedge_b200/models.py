@@ -807,6 +807,14 @@ class VariableCoefficientAdvectionOperator(HyperbolicOperator):
         return float(np.sqrt(np.max(np.sum(v.reshape(self.dimensions, -1) ** 2, axis=0))))
 
 
+# the given functions that each model's own ``context`` evaluates
+CONTEXT_DATA = {
+    StrongAdvectionOperator.context: ("inflow_u",),
+    StrongWaveOperator.context: ("dirichlet_bc_f",),
+    VariableCoefficientAdvectionOperator.context: ("advec_v", "bc_u_f"),
+}
+
+
 def _template_value(x, name):
     """A model datum as a template term: expressions and numbers as they
     are, volume vectors as the field ``name`` (bound when the model binds)."""
