@@ -33,6 +33,17 @@ RK4C = [0.0,
 
 # the same for the native step
 _A, _B = (C.c_double * 5)(*RK4A), (C.c_double * 5)(*RK4B)
+_TABLE = np.array([RK4A, RK4B, RK4C], dtype=np.float64).T
+_TABLE_BYTES = _TABLE.tobytes()
+
+
+def _stage_arrays(coeffs):
+    """The a and b columns of a coefficient table for the native step."""
+    table = np.asarray(coeffs, dtype=np.float64)
+    if table.tobytes() == _TABLE_BYTES:
+        return _A, _B
+    a, b, _ = table.T.tolist()
+    return (C.c_double * len(a))(*a), (C.c_double * len(b))(*b)
 
 
 class LSRK4TimeStepper:
@@ -41,7 +52,7 @@ class LSRK4TimeStepper:
 
     def __init__(self, dtype=np.float64, rcon=None, vector_primitive_factory=None):
         self.dtype = np.dtype(dtype)
-        self.coeffs = np.array([RK4A, RK4B, RK4C], dtype=np.float64).T
+        self.coeffs = _TABLE.copy()
         self.residual = None
 
     def __call__(self, y, t, dt, rhs):
@@ -56,10 +67,11 @@ class LSRK4TimeStepper:
             # written (the reference also returns a new state each step)
             bufs = [torch.empty_like(y), torch.empty_like(y)]
             if rhs.constant_context():
-                # the model's data evaluated once, the five stages in one call
-                comp.lsrk_step(_A, _B, dt, [y, bufs[0], bufs[1], bufs[0], bufs[1], bufs[0]],
-                               self.residual, **rhs.context(t))
-                return bufs[0]
+                # the model's data evaluated once, the stages in one call
+                a, b = _stage_arrays(self.coeffs)
+                stages = [y] + [bufs[s % 2] for s in range(len(a))]
+                comp.lsrk_step(a, b, dt, stages, self.residual, **rhs.context(t))
+                return stages[-1]
             cur = y
             for s, (a, b, c) in enumerate(self.coeffs):
                 nxt = bufs[s % 2]

@@ -102,6 +102,16 @@ def test_known_constant_data(model, make):
     assert [s[:2] for s in comp.stages] == list(zip(RK4A, RK4B))
 
 
+@pytest.mark.parametrize("data", [CONST(ONE), CHANGING(TIME)])
+@pytest.mark.parametrize("n", [4, 5])
+def test_the_steppers_own_coefficients(data, n):
+    comp = _Recorder(MODEL_ADVECTION)
+    stepper = hb.LSRK4TimeStepper()
+    stepper.coeffs = np.linspace(0.1, 0.9, 3 * n).reshape(n, 3)
+    stepper(torch.zeros(1, 4), 0.25, 0.5, BoundRHS(comp, _advection(data)))
+    assert [s[:2] for s in comp.stages] == [(a, b) for a, b, _ in stepper.coeffs]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("which", ["advection", "maxwell", "any object"])
 def test_step_equals_stages(cuda_device, which):
