@@ -705,13 +705,26 @@ class CompiledOperator:
         arrays of doubles) in one native call; boundary values, coefficient
         and, unless ``source_stride`` (values between the stages' sources)
         is given, source hold for all of them."""
+        n = len(a)
+        if len(b) != n or len(bufs) != n + 1 or \
+                any(getattr(x, "_type_", None) is not C.c_double for x in (a, b)):
+            raise ValueError("%d stages need %d coefficients a and b (ctypes doubles) and %d "
+                             "buffers" % (n, n, n + 1))
         keep, bptr = self._bdry_ptr(bc_in)
         if source_stride:
+            rows = (self._n_e or 1) * len(self.discr)
+            if self.var_material:
+                raise ValueError("variable material: one source for all stages")
+            if source_stride < 0 or source.dtype != _torch().float64 or \
+                    not source.is_contiguous() or source.device != self.discr.device or \
+                    source.numel() < (n - 1) * source_stride + rows:
+                raise ValueError("source: contiguous FP64 on the device, stage s's %d values "
+                                 "from s * source_stride" % rows)
             cptr, sptr = self._field_ptrs(coeff, None)[0], source.data_ptr()
         else:
             cptr, sptr = self._field_ptrs(coeff, source)
         _native.check(self._lib.hb_lsrk_step(
-            self._handle, len(a), a, b, float(dt),
+            self._handle, n, a, b, float(dt),
             (C.c_void_p * len(bufs))(*[x.data_ptr() for x in bufs]), res.data_ptr(), cptr, bptr,
             sptr, source_stride, self._stream()))
 

@@ -1,0 +1,83 @@
+"""CompiledOperator hands raw pointers to the native library: what does not fit
+is refused before the call.  On the CPU, with a stand-in for the library."""
+import ctypes as C
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from hedge_b200.discretization import CompiledOperator
+from hedge_b200.models import MODEL_VARWAVE
+
+N, F = 12, 3
+
+
+class _Discr(SimpleNamespace):
+    def __len__(self):
+        return N
+
+
+class _Library:
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        return lambda *args: self.calls.append((name, args)) or 0
+
+
+def _operator(**kw):
+    op = CompiledOperator.__new__(CompiledOperator)
+    op.__dict__.update(discr=_Discr(device=torch.device("cpu"), dimensions=2), F=F, n_given=0,
+                       ot=SimpleNamespace(model=MODEL_VARWAVE), var_material=False, _n_e=0,
+                       _coeff=torch.ones(N, dtype=torch.float64), _source=None, _handle=None,
+                       _lib=_Library(), _stream=lambda: 0,
+                       _adj_work=torch.empty(4, dtype=torch.float64))
+    op.__dict__.update(kw)
+    return op
+
+
+def _vec(*shape, dtype=torch.float64):
+    return torch.ones(shape, dtype=dtype)
+
+
+def _doubles(n):
+    return (C.c_double * n)(*range(n))
+
+
+def test_step_takes_a_complete_stage_list():
+    op = _operator()
+    op.lsrk_step(_doubles(2), _doubles(2), 0.1, [_vec(F, N) for _ in range(3)], _vec(F, N),
+                 source=_vec(2, N), source_stride=N)
+    assert [c[0] for c in op._lib.calls] == ["hb_lsrk_step"]
+
+
+@pytest.mark.parametrize("a,b,buffers,kw", [
+    (2, 2, 2, {}), (2, 1, 3, {}), (1, 2, 3, {}),
+    (2, 2, 3, dict(source=_vec(N + 1), source_stride=N)),
+    (2, 2, 3, dict(source=_vec(2, N, dtype=torch.float32), source_stride=N)),
+    (2, 2, 3, dict(source=_vec(N, 2).T, source_stride=N)),
+    (2, 2, 3, dict(source=_vec(2, N), source_stride=-N)),
+])
+def test_step_refuses(a, b, buffers, kw):
+    op = _operator()
+    with pytest.raises(ValueError):
+        op.lsrk_step(_doubles(a), _doubles(b), 0.1, [_vec(F, N) for _ in range(buffers)],
+                     _vec(F, N), **kw)
+    assert not op._lib.calls
+
+
+def test_step_refuses_other_coefficient_types():
+    op = _operator()
+    with pytest.raises(ValueError):
+        op.lsrk_step((C.c_float * 2)(), _doubles(2), 0.1, [_vec(F, N) for _ in range(3)],
+                     _vec(F, N))
+    assert not op._lib.calls
+
+
+def test_step_refuses_stage_sources_with_variable_material():
+    # the material divides a source before the kernel sees it
+    op = _operator(var_material=True, _n_e=3, _coeff=_vec(2 * N))
+    with pytest.raises(ValueError):
+        op.lsrk_step(_doubles(2), _doubles(2), 0.1, [_vec(F, N) for _ in range(3)], _vec(F, N),
+                     source=_vec(2, 3 * N), source_stride=3 * N)
+    assert not op._lib.calls
