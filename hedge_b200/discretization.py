@@ -752,10 +752,10 @@ class CompiledOperator:
 
     def _adjoint_work(self):
         torch = _torch()
-        nbytes = C.c_int64()
-        _native.check(self._lib.hb_rhs_adjoint_work_size(self._handle, C.byref(nbytes)))
         work = getattr(self, "_adj_work", None)
-        if work is None or work.numel() * 8 < nbytes.value:
+        if work is None:
+            nbytes = C.c_int64()
+            _native.check(self._lib.hb_rhs_adjoint_work_size(self._handle, C.byref(nbytes)))
             work = torch.empty((nbytes.value + 7) // 8, dtype=torch.float64,
                                device=self.discr.device)
             self._adj_work = work
@@ -769,9 +769,20 @@ class CompiledOperator:
             lam += b lq;  lq += dt (dR/dq)^T lam;  c_bar += dt (dR/dc)^T lam;
             lam *= a
 
-        (hb_adjoint_stage: two launches; where that refuses, beyond order 7,
-        composed from ``adjoint``)."""
+        with the state q [F, K*Np] of any real type (hb_adjoint_stage: two
+        launches; where that refuses, beyond order 7, composed from
+        ``adjoint``)."""
+        d = self.discr
+        n, f64 = len(d), _torch().float64
         c = self._coeff if coeff is None else coeff
+        for name, x, size in (("lam", lam, self.F * n), ("lq", lq, self.F * n),
+                              ("c_bar", c_bar, n), ("coeff", coeff, n)):
+            if x is not None and (x.dtype != f64 or not x.is_contiguous() or
+                                  x.numel() != size or x.device != d.device):
+                raise ValueError("%s: contiguous FP64 [%d] on the device" % (name, size))
+        if q is not None and (q.dtype != f64 or not q.is_contiguous() or
+                              q.numel() != self.F * n or q.device != d.device):
+            q = q.to(device=d.device, dtype=f64).reshape(self.F, n).contiguous()
         st = self._lib.hb_adjoint_stage(
             self._handle, float(a), float(b), float(dt),
             q.data_ptr() if q is not None else None, lam.data_ptr(), lq.data_ptr(),
@@ -781,11 +792,12 @@ class CompiledOperator:
         if st != _native.HB_ERR_UNSUPPORTED:
             _native.check(st)
             return
+        lam, lq = lam.view(self.F, n), lq.view(self.F, n)
         lam.add_(lq, alpha=b)
         q_bar, cb = self.adjoint(lam, q=q, coeff=coeff, want_c=c_bar is not None)
         lq.add_(q_bar, alpha=dt)
         if c_bar is not None:
-            c_bar.add_(cb, alpha=dt)
+            c_bar.view(n).add_(cb, alpha=dt)
         lam.mul_(a)
 
     def check(self):

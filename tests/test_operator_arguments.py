@@ -81,3 +81,39 @@ def test_step_refuses_stage_sources_with_variable_material():
         op.lsrk_step(_doubles(2), _doubles(2), 0.1, [_vec(F, N) for _ in range(3)], _vec(F, N),
                      source=_vec(2, 3 * N), source_stride=3 * N)
     assert not op._lib.calls
+
+
+def test_adjoint_stage_takes_device_vectors():
+    op = _operator()
+    q = _vec(F, N, dtype=torch.float32)          # converted, as adjoint() does
+    op.adjoint_stage(0.1, 0.2, 0.3, _vec(F, N), _vec(F * N), q=q, c_bar=_vec(N))
+    (name, args), = op._lib.calls
+    assert name == "hb_adjoint_stage" and args[4] not in (None, q.data_ptr())
+
+
+@pytest.mark.parametrize("bad", [_vec(F, N, dtype=torch.float32), _vec(F, N - 1), _vec(N, F).T,
+                                 _vec(F, 2 * N)[:, ::2], torch.ones(1, 1).double().expand(F, N)])
+@pytest.mark.parametrize("which", ["lam", "lq"])
+def test_adjoint_stage_refuses_vectors(which, bad):
+    op = _operator()
+    x = dict(lam=_vec(F, N), lq=_vec(F, N), q=_vec(F, N))
+    x[which] = bad
+    with pytest.raises(ValueError):
+        op.adjoint_stage(0.1, 0.2, 0.3, **x)
+    assert not op._lib.calls
+
+
+@pytest.mark.parametrize("which", ["c_bar", "coeff"])
+@pytest.mark.parametrize("bad", [_vec(N, dtype=torch.float32), _vec(N - 1), _vec(2 * N)[::2]])
+def test_adjoint_stage_refuses_coefficients(which, bad):
+    op = _operator()
+    with pytest.raises(ValueError):
+        op.adjoint_stage(0.1, 0.2, 0.3, _vec(F, N), _vec(F, N), q=_vec(F, N), **{which: bad})
+    assert not op._lib.calls
+
+
+def test_adjoint_stage_refuses_a_short_state():
+    op = _operator()
+    with pytest.raises(RuntimeError):
+        op.adjoint_stage(0.1, 0.2, 0.3, _vec(F, N), _vec(F, N), q=_vec(F, N - 1))
+    assert not op._lib.calls
