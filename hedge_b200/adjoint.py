@@ -190,8 +190,12 @@ class ReceiverTraces:
                     cc = cc if ctx.has_c else None
                     comp, rec, dt = ctx.comp, ctx.receivers, ctx.dt
                     want_c = ctx.has_c and ctx.needs_input_grad[1]
+                    # lq is updated in place: an FP64 copy of its own, whatever
+                    # the receivers return
                     q_last = ctx.checkpoints[0]
                     lq = rec.transpose(g[ctx.nsteps], q_last)
+                    lq = torch.empty(q_last.shape, dtype=torch.float64,
+                                     device=q_last.device).copy_(lq)
                     c_bar = torch.zeros_like(cc) if want_c else None
                     starts = sorted(ctx.checkpoints)
                     ends = starts[1:] + [ctx.nsteps]
@@ -214,7 +218,7 @@ class ReceiverTraces:
                             for s in range(4, -1, -1):
                                 comp.adjoint_stage(RK4A[s], RK4B[s], dt, lres, lq,
                                                    q=keep[s], coeff=cc, c_bar=c_bar)
-                            lq = lq + rec.transpose(g[n], lq)
+                            lq = (lq + rec.transpose(g[n], lq)).contiguous()
                     q0_bar = lq.reshape(ctx.checkpoints[0].shape)
                     return q0_bar, c_bar, None, None, None, None, None, None
 
