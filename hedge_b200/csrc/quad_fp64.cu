@@ -113,7 +113,8 @@ __global__ void __launch_bounds__(QUAD_THREADS) quad_fp64_kernel(const QuadF64Ar
           double s = 0.0;
 #pragma unroll
           for (int x = 0; x < DIM; ++x) s += rx[r][x] * c[1 + x][h];
-          gr[h] = c[0][h] * s;
+          // (points beyond the last are 0 * w, not zero where w is not finite)
+          gr[h] = 8 * qt + 2 * t + h < a.nq ? c[0][h] * s : 0.0;
         }
 #pragma unroll
         for (int m = 0; m < KS; ++m) {
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(QUAD_THREADS) quad_fp64_kernel(const QuadF64Ar
           v = 0.5 * (nvm * cm[0][h] + nvp * cp[0][h]) - 0.5 * (cp[0][h] - cm[0][h]) * cmax;
         else
           v = navg > 0.0 ? nvm * cm[0][h] : nvp * cp[0][h];
-        fl[h] = none ? 0.0 : fscale * v;
+        fl[h] = none || 8 * pt + 2 * t + h >= a.nqf ? 0.0 : fscale * v;
       }
 #pragma unroll
       for (int m = 0; m < KS; ++m) {
