@@ -4,16 +4,19 @@
 //
 //   adj_lift_kernel     W[e][p][f] = Fscale s_f sum_i LIFT[i][p] lam_f[i]
 //                       (s_f the model's output scale), M = face points;
-//   adj_element_kernel  q_bar = [ D_1^T .. D_d^T | I_face ] . [ y_1; ..; y_d; w ]
-//                       with y_r the transposed chain rule and volume map of
-//                       s_f lam_f at the nodes, w the transposed fluxes of
-//                       both sides at the face points (the neighbour's from
-//                       its W: a gather, no atomics) and I_face the 0/1
-//                       matrix that adds a face point to its volume node.
+//   adj_element_kernel  q_bar = [ D_1^T .. D_d^T ] . [ y_1; ..; y_d ] + w at
+//                       the face points' nodes, with y_r the transposed chain
+//                       rule and volume map of s_f lam_f at the nodes and w
+//                       the transposed fluxes of both sides at the face
+//                       points (the neighbour's from its W: a gather, no
+//                       atomics).  The output pass adds a node's face points
+//                       from a list: as one more block of the product, a 0/1
+//                       matrix, a w that is not finite would make every node
+//                       of the element NaN.
 //
 // The c gradient of the variable-velocity wave rides along: the face part is
-// one more column per element, the volume part sum_f s_f lam_f vol_f(grad q,
-// c = 1) a second contraction with the forward derivatives.
+// one more row of w, the volume part sum_f s_f lam_f vol_f(grad q, c = 1) a
+// second contraction with the forward derivatives.
 //
 // Either kernel may also carry one step of the reversed LSRK recurrences
 //   lam <- lam + b lq;  lq <- lq + dt (dR/dq)^T lam;  c_bar <- c_bar + dt
@@ -66,18 +69,18 @@ struct AdjShape : F64Shape<MODEL, DIM, ORDER> {
   using B::F; using B::C; using B::NP; using B::NFP; using B::NF; using B::NFPT; using B::G;
   using B::KV; using B::MT; using B::RN; using B::NGW; using B::KG; using B::THREADS;
   using B::COLS; using B::LDP;
-  // columns per element: the fields, and the c gradient's face part
+  // values per face point: the fields, and the c gradient's
   static constexpr int CF = F + (WC ? 1 : 0);
   static constexpr int EB = COLS / CF;
-  static constexpr int KP = f64_ru8(KV + NFPT);
-  static constexpr int STEPS = KP / 8;
-  static constexpr int VSTEPS = f64_ru8(KV) / 8;   // of the forward derivatives
+  static constexpr int KP = f64_ru8(KV);
+  static constexpr int STEPS = KP / 8;             // of either direction's derivatives
   static constexpr int LDZ = KP % 16 == 8 ? KP : KP + 8;
   static constexpr int ENP = EB * NP;
   static constexpr size_t al(size_t x) { return (x + 15) & ~size_t(15); }
   static constexpr size_t zdoubles =
       COLS * LDZ > KG * COLS * LDP ? COLS * LDZ : KG * COLS * LDP;
-  static constexpr size_t oL = al(8 * zdoubles);               // [F][EB][NP] s_f lam_f
+  static constexpr size_t oW = al(8 * zdoubles);               // [EB][CF][NFPT] w
+  static constexpr size_t oL = al(oW + 8 * EB * CF * NFPT);    // [F][EB][NP] s_f lam_f
   static constexpr size_t oQ = al(oL + 8 * F * ENP);           // [F][EB][NP] state (WC)
   static constexpr size_t oC = al(oQ + (WC ? 8 * F * ENP : 0));   // [EB][NP]
   static constexpr size_t oV = al(oC + 8 * C * ENP);           // [EB][NP] volume c part
@@ -85,7 +88,9 @@ struct AdjShape : F64Shape<MODEL, DIM, ORDER> {
   static constexpr size_t oN = al(oG + 8 * EB * G);
   static constexpr size_t oFm = al(oN + 8 * EB * NF);
   static constexpr size_t oSh = al(oFm + NFPT);                // shuffle
-  static constexpr size_t total = al(oSh + 6 * NFP);
+  static constexpr int NLIST = NP + 1 + NFPT;
+  static constexpr size_t oNl = al(oSh + 6 * NFP);             // nodes' face points
+  static constexpr size_t total = al(oNl + NLIST);
   // lift pass: M = face points, the row tiles split over the warps
   static constexpr int LW = 4;
   static constexpr int LMT = (NFPT + 7) / 8;
@@ -105,8 +110,9 @@ struct AdjArgs {
   int64_t K, nbatch;
   int E, nperm;
   const double2* lfrag;      // LIFT^T fragments [LSTEPS][LW * LMW][32]
-  const double2* afrag;      // [D^T | I_face] fragments
+  const double2* afrag;      // [D^T] fragments
   const double2* vfrag;      // [D] fragments (c gradient)
+  const uint8_t* nlist;      // [np + 1] begins of the nodes' face points, the face points
   const double* geo;
   const int2* conn;
   const int* fmask;
@@ -211,16 +217,20 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
   int2* sconn = reinterpret_cast<int2*>(smem + S::oN);
   uint8_t* sfm = smem + S::oFm;
   uint8_t* ssh = smem + S::oSh;
+  uint8_t* snl = smem + S::oNl;
+  double* sw = reinterpret_cast<double*>(smem + S::oW);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int kg = warp % KG, ng = warp / KG;
   const int64_t Knp = a.K * NP;
   for (int x = tid; x < NFPT; x += THREADS) sfm[x] = (uint8_t)a.fmask[x];
   for (int x = tid; x < a.nperm * NFP; x += THREADS) ssh[x] = (uint8_t)a.shuffle[x];
+  for (int x = tid; x < S::NLIST; x += THREADS) snl[x] = a.nlist[x];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // GEMM of `steps` steps over the columns [0, cols), partial sums into Z
-  auto gemm = [&](const double2* frag, int steps, int cols) {
+  // product with a derivative operator over the columns [0, cols), partial
+  // sums into Z
+  auto gemm = [&](const double2* frag, int cols) {
     const bool work = ng * RN * 8 < cols;
     double acc[MT][RN][2];
 #pragma unroll
@@ -228,7 +238,7 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
 #pragma unroll
       for (int c = 0; c < RN; ++c) acc[m][c][0] = acc[m][c][1] = 0.0;
     if (work) {
-      const int s0 = kg * steps / KG, s1 = (kg + 1) * steps / KG;
+      const int s0 = kg * S::STEPS / KG, s1 = (kg + 1) * S::STEPS / KG;
       dmma_steps<MT, RN, LDZ>(
           acc, frag + (size_t)s0 * MT * 32 + lane,
           sZ + (ng * RN * 8 + (lane >> 2)) * LDZ + 2 * (lane & 3) + 8 * s0, s1 - s0);
@@ -247,10 +257,10 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
     }
     __syncthreads();
   };
-  // rows [k0, k1), fewer than 8, of the columns [0, cols)
-  auto zero_rows = [&](int k0, int k1, int cols) {
+  // the rows that pad a column of Z, fewer than 8
+  auto zero_rows = [&](int cols) {
     for (int x = tid; x < cols * 8; x += THREADS)
-      if (k0 + x % 8 < k1) sZ[(x / 8) * LDZ + k0 + x % 8] = 0.0;
+      if (KV + x % 8 < S::KP) sZ[(x / 8) * LDZ + KV + x % 8] = 0.0;
   };
   auto sum = [&](int col, int i) {
     double v = sZ[col * S::LDP + i];
@@ -296,9 +306,9 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
           for (int f = 0; f < F; ++f) z[f * LDZ + r * NP] = vol[f];
         }
       }
-      zero_rows(KV, S::VSTEPS * 8, ne * F);
+      zero_rows(ne * F);
       __syncthreads();
-      gemm(a.vfrag, S::VSTEPS, ne * F);
+      gemm(a.vfrag, ne * F);
       for (int x = tid; x < ne * NP; x += THREADS) {
         const int e = x / NP, i = x - e * NP;
         double s = 0.0;
@@ -335,9 +345,9 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
           m[d][g] = s;
         }
       const double* ge = sgeo + e * G;
-      double* z = sZ + e * CF * LDZ + i;
+      double* z = sZ + e * F * LDZ + i;
 #pragma unroll
-      for (int r = 0; r < DIM; ++r) {
+      for (int r = 0; r < DIM; ++r)
 #pragma unroll
         for (int g = 0; g < F; ++g) {
           double s = 0.0;
@@ -345,10 +355,8 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
           for (int d = 0; d < DIM; ++d) s += ge[r * DIM + d] * m[d][g];
           z[g * LDZ + r * NP] = s;
         }
-        if constexpr (WC) z[F * LDZ + r * NP] = 0.0;
-      }
     }
-    zero_rows(KV + NFPT, S::KP, ne * CF);
+    zero_rows(ne * F);
     // ---- transposed own-side and neighbour-side fluxes at the face points ----
     for (int it = tid; it < ne * NFPT; it += THREADS) {
       const int e = it / NFPT, p = it - e * NFPT, face = p / NFP, k = p - face * NFP;
@@ -384,7 +392,7 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
         nnb[d] = nb >= 0 ? __ldg(a.geo + nb * G + DIM * DIM + (cn.y & 3) * (DIM + 1) + d) : 0.0;
       const double cm = C ? sc[e * NP + lnode] : 0.0;
       const double cp = (C && nb >= 0) ? __ldg(a.coeff + nb * NP + nn) : cm;
-      double* z = sZ + e * CF * LDZ + KV + p;
+      double* w = sw + e * CF * NFPT + p;
 #pragma unroll
       for (int g = 0; g < F; ++g) {
         double uM[NA], uP[NA], fl[F];
@@ -407,7 +415,7 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
 #pragma unroll
           for (int f = 0; f < F; ++f) s += wn[f] * fl[f];
         }
-        z[g * LDZ] = s;
+        w[g * NFPT] = s;
       }
       if constexpr (WC) {
         double uM[NA], uP[NA], fl[F], gc = 0.0;
@@ -435,18 +443,21 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
 #pragma unroll
           for (int f = 0; f < F; ++f) gc += wn[f] * fl[f];
         }
-        z[F * LDZ] = gc;
+        w[F * NFPT] = gc;
       }
     }
     __syncthreads();
-    gemm(a.afrag, S::STEPS, ne * CF);
+    gemm(a.afrag, ne * F);
 
     // ---- output ----
     for (int x = tid; x < ne * NP; x += THREADS) {
       const int e = x / NP, i = x - e * NP;
+      const double* w = sw + e * CF * NFPT;
+      const int p0 = snl[i], p1 = snl[i + 1];
 #pragma unroll
       for (int g = 0; g < F; ++g) {
-        const double v = sum(e * CF + g, i);
+        double v = sum(e * F + g, i);
+        for (int p = p0; p < p1; ++p) v += w[g * NFPT + snl[NP + 1 + p]];
         const int64_t gi = g * Knp + el0 * NP + x;
         if (a.fused) {
           a.lq[gi] += a.dt * v;
@@ -456,7 +467,8 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
         }
       }
       if constexpr (WC) {
-        const double v = sum(e * CF + F, i) + sv[x];
+        double v = sv[x];
+        for (int p = p0; p < p1; ++p) v += w[F * NFPT + snl[NP + 1 + p]];
         const int64_t gi = el0 * NP + x;
         if (a.fused)
           a.c_bar[gi] += a.dt * v;
@@ -475,7 +487,8 @@ struct AdjCall {
   bool configure;
 };
 
-// The operator fragments of the adjoint: [LIFT^T | D^T, I_face | D].
+// The operator fragments of the adjoint, [LIFT^T | D^T | D], and the nodes'
+// face points.
 template <int MODEL, int DIM, int ORDER>
 hb_status adj_fragments(Op* op) {
   using S = AdjShape<MODEL, DIM, ORDER, false>;
@@ -483,8 +496,7 @@ hb_status adj_fragments(Op* op) {
   const double* h = reinterpret_cast<const double*>(d->host_blob.data());
   const double* lift = h + (size_t)DIM * S::NP * S::NP;
   const size_t nl = (size_t)S::LW * S::LSTEPS * S::LMW * 64, na = (size_t)S::STEPS * S::MT * 64;
-  const size_t nv = (size_t)S::VSTEPS * S::MT * 64;
-  std::vector<double> fr(nl + na + nv, 0.0);
+  std::vector<double> fr(nl + 2 * na + (S::NLIST + 7) / 8, 0.0);
   for (int p = 0; p < S::NFPT; ++p)
     for (int i = 0; i < S::NP; ++i) {
       const int w = p / (S::LMW * 8), row = p - w * S::LMW * 8;
@@ -501,7 +513,15 @@ hb_status adj_fragments(Op* op) {
       }
   std::vector<int> fm(S::NFPT);
   HB_CUDA(cudaMemcpy(fm.data(), d->fmask, sizeof(int) * S::NFPT, cudaMemcpyDeviceToHost));
-  for (int p = 0; p < S::NFPT; ++p) fr[nl + dmma_afrag(fm[p], S::KV + p, S::MT)] = 1.0;
+  uint8_t* begin = reinterpret_cast<uint8_t*>(&fr[nl + 2 * na]);
+  uint8_t* list = begin + S::NP + 1;
+  int n = 0;
+  for (int i = 0; i < S::NP; ++i) {
+    begin[i] = (uint8_t)n;
+    for (int p = 0; p < S::NFPT; ++p)
+      if (fm[p] == i) list[n++] = (uint8_t)p;
+  }
+  begin[S::NP] = (uint8_t)n;
   double* dev = nullptr;
   if (cudaMalloc(&dev, sizeof(double) * fr.size()) != cudaSuccess)
     return fail(HB_ERR_CUDA, "cannot allocate the adjoint's operator fragments");
@@ -548,6 +568,8 @@ hb_status adj_one(const AdjCall& c) {
   using S = AdjShape<MODEL, DIM, ORDER, false>;
   constexpr bool CW = S::C != 0;
   using SC = AdjShape<MODEL, DIM, ORDER, CW>;
+  static_assert(SC::total <= 227 * 1024 && S::total <= 227 * 1024 && S::ltotal <= 227 * 1024,
+                "a batch exceeds the shared memory of a CTA");
   Op* op = c.op;
   const Discr* d = op->d;
   if (d->np != S::NP || d->nfp != S::NFP)
@@ -570,6 +592,7 @@ hb_status adj_one(const AdjCall& c) {
   a.lfrag = reinterpret_cast<const double2*>(op->adjfrag);
   a.afrag = a.lfrag + (size_t)S::LW * S::LSTEPS * S::LMW * 32;
   a.vfrag = a.afrag + (size_t)S::STEPS * S::MT * 32;
+  a.nlist = reinterpret_cast<const uint8_t*>(a.vfrag + (size_t)S::STEPS * S::MT * 32);
   a.geo = d->geo;
   a.conn = op->conn;
   a.fmask = d->fmask;
@@ -582,7 +605,7 @@ hb_status adj_one(const AdjCall& c) {
                                   op->adj_slots[0], c.stream);
   if (st) return st;
   const int slots = op->adj_slots[wc ? 2 : 1];
-  a.E = dmma_batch(d->K, wc ? SC::EB : S::EB, wc ? SC::CF : S::CF, slots);
+  a.E = dmma_batch(d->K, wc ? SC::EB : S::EB, S::F, slots);
   a.nbatch = (d->K + a.E - 1) / a.E;
   if constexpr (CW) {
     if (wc)

@@ -1,8 +1,8 @@
 """A value that is not finite reaches only what depends on it.  The result is
 formed with two finite values in one element first: what does not change
 between them does not depend on that element, and stays bit for bit as it is
-with infinities and NaN there (the padding of a tile must not
-spread them)."""
+with infinities and NaN there (neither the padding of a tile
+nor a product with a 0/1 matrix may spread them)."""
 import numpy as np
 import pytest
 
@@ -67,3 +67,41 @@ def test_quadrature_upwind(cuda_device, dim, order, degree, precision):
     kept = [bool(same.reshape(d.K, d.Np)[k].all()) for k in neighbours]
     assert any(kept) and not all(kept)
     rhs.compiled.check()
+
+
+@pytest.mark.parametrize("order", [1, 3, 5, 7, 8])
+@pytest.mark.parametrize("model,dim", [("advection", 2), ("varwave", 2), ("wave", 3),
+                                       ("varwave", 3), ("maxwell", 3), ("tm", 2)])
+def test_adjoint(cuda_device, model, dim, order):
+    """The cotangent in an element, and the state for the c gradient, reach the
+    neighbours' nodes on the shared faces and no others (orders 1 to 7 and the
+    CUDA-core kernel beyond)."""
+    import torch
+    from test_gpu_fp64_tensor import _mesh as tagged, _operator
+    mesh = tagged(dim, 5, 5) if dim == 2 else tagged(dim, 2, 2)
+    d = hb.Discretization(mesh, order=order)
+    op = _operator(model, dim, d)
+    comp = d.compile(op.op_template())
+    e = _inner(d)
+    mine = torch.zeros(len(d), dtype=torch.bool, device=d.device)
+    mine[e * d.Np:(e + 1) * d.Np] = True
+    inner, outer = comp.gather_map()
+    reached = mine.clone()
+    inside = outer >= 0
+    reached[inner[inside][mine[outer[inside]]]] = True
+    assert int(reached.sum()) > d.Np
+    rng = np.random.default_rng(order)
+    q, lam = (d.to_device(rng.uniform(-1, 1, (comp.F, len(d)))) for _ in range(2))
+    want_c = model == "varwave"
+    q_bar, c_bar = comp.adjoint(lam, q=q, want_c=want_c)
+    for bad in (float("inf"), float("nan")):
+        x = torch.where(mine, bad, lam)
+        got, _ = comp.adjoint(x, q=q)
+        assert torch.equal(got[:, ~reached], q_bar[:, ~reached])
+        assert not bool(torch.isfinite(got[:, mine]).all())
+        if want_c:
+            for l, s in ((x, q), (lam, torch.where(mine, bad, q))):
+                _, got = comp.adjoint(l, q=s, want_c=True)
+                assert torch.equal(got[~reached], c_bar[~reached])
+                assert not bool(torch.isfinite(got[mine]).all())
+    comp.check()
