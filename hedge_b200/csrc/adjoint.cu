@@ -340,7 +340,7 @@ int64_t adjoint_work_bytes(const Op* op) {
 
 hb_status launch_adjoint(Op* op, const double* q, const double* lam, double* q_bar,
                          double* c_bar, const double* coeff, double* work, cudaStream_t s) {
-  if (adjoint_f64_ready(op, s))
+  if (adjoint_f64_ready(op, c_bar != nullptr, s))
     return launch_adjoint_f64(op, q, lam, q_bar, c_bar, coeff, work, s);
   const int dim = op->d->dim;
   switch (op->model) {

@@ -25,27 +25,32 @@ static hb_status adj_dispatch(const AdjCall& c) {
   }
 }
 
-bool adjoint_f64_ready(Op* op, cudaStream_t s) {
-  const int state = op->adj_state.load(std::memory_order_acquire);
-  if (state) return state == 1;
+bool adjoint_f64_ready(Op* op, bool want_c, cudaStream_t s) {
+  const int variant = want_c ? 1 : 0;
+  if (op->adj.has(variant)) return true;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (op->d->order > 7 || cudaStreamIsCapturing(s, &cap) != cudaSuccess ||
       cap != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
     return false;
   }
-  std::lock_guard<std::mutex> lock(op->adj_mutex);
-  if (op->adj_state.load(std::memory_order_acquire) == 0) {
-    // (allocating here must not upset a capture on another thread)
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    AdjCall c = {};
-    c.op = op;
-    c.configure = true;
-    op->adj_state.store(adj_dispatch(c) == HB_OK ? 1 : 2, std::memory_order_release);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-  }
-  return op->adj_state.load(std::memory_order_acquire) == 1;
+  // (allocating here must not upset a capture on another thread)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const bool ok = op->adj.ready(
+      variant,
+      [&]() {
+        AdjCall c = {};
+        c.op = op;
+        c.stream = s;
+        c.configure = true;
+        c.want_c = want_c;
+        return adj_dispatch(c);
+      },
+      // the CUDA-core adjoint's launches ask for the last error
+      []() { cudaGetLastError(); });
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return ok;
 }
 
 hb_status launch_adjoint_f64(Op* op, const double* q, const double* lam, double* q_bar,

@@ -484,19 +484,20 @@ struct AdjCall {
   Op* op;
   AdjArgs a;
   cudaStream_t stream;
-  bool configure;
+  bool configure, want_c;   // prepare the operator, without or with the c gradient
 };
 
-// The operator fragments of the adjoint, [LIFT^T | D^T | D], and the nodes'
-// face points.
+// The operator fragments of the adjoint, [LIFT^T | D^T | D], D where there is
+// a c gradient, and the nodes' face points.
 template <int MODEL, int DIM, int ORDER>
-hb_status adj_fragments(Op* op) {
+hb_status adj_fragments(Op* op, cudaStream_t s) {
   using S = AdjShape<MODEL, DIM, ORDER, false>;
   const Discr* d = op->d;
   const double* h = reinterpret_cast<const double*>(d->host_blob.data());
   const double* lift = h + (size_t)DIM * S::NP * S::NP;
   const size_t nl = (size_t)S::LW * S::LSTEPS * S::LMW * 64, na = (size_t)S::STEPS * S::MT * 64;
-  std::vector<double> fr(nl + 2 * na + (S::NLIST + 7) / 8, 0.0);
+  const size_t ops = nl + (S::C ? 2 : 1) * na;
+  std::vector<double> fr(ops + (S::NLIST + 7) / 8, 0.0);
   for (int p = 0; p < S::NFPT; ++p)
     for (int i = 0; i < S::NP; ++i) {
       const int w = p / (S::LMW * 8), row = p - w * S::LMW * 8;
@@ -509,24 +510,24 @@ hb_status adj_fragments(Op* op) {
       for (int j = 0; j < S::NP; ++j) {
         const double v = h[((size_t)r * S::NP + j) * S::NP + i];
         fr[nl + dmma_afrag(j, r * S::NP + i, S::MT)] = v;
-        fr[nl + na + dmma_afrag(i, r * S::NP + j, S::MT)] = v;
+        if (S::C) fr[nl + na + dmma_afrag(i, r * S::NP + j, S::MT)] = v;
       }
-  std::vector<int> fm(S::NFPT);
-  HB_CUDA(cudaMemcpy(fm.data(), d->fmask, sizeof(int) * S::NFPT, cudaMemcpyDeviceToHost));
-  uint8_t* begin = reinterpret_cast<uint8_t*>(&fr[nl + 2 * na]);
+  uint8_t* begin = reinterpret_cast<uint8_t*>(&fr[ops]);
   uint8_t* list = begin + S::NP + 1;
   int n = 0;
   for (int i = 0; i < S::NP; ++i) {
     begin[i] = (uint8_t)n;
     for (int p = 0; p < S::NFPT; ++p)
-      if (fm[p] == i) list[n++] = (uint8_t)p;
+      if (d->fmask_host[p] == i) list[n++] = (uint8_t)p;
   }
   begin[S::NP] = (uint8_t)n;
   double* dev = nullptr;
   if (cudaMalloc(&dev, sizeof(double) * fr.size()) != cudaSuccess)
     return fail(HB_ERR_CUDA, "cannot allocate the adjoint's operator fragments");
-  if (cudaMemcpy(dev, fr.data(), sizeof(double) * fr.size(), cudaMemcpyHostToDevice) !=
-      cudaSuccess) {
+  // waited for: another thread's stream may be the next to read it
+  if (cudaMemcpyAsync(dev, fr.data(), sizeof(double) * fr.size(), cudaMemcpyHostToDevice, s) !=
+          cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess) {
     cudaFree(dev);
     return fail(HB_ERR_CUDA, "cannot upload the adjoint's operator fragments");
   }
@@ -553,6 +554,7 @@ hb_status adj_launch(KERN kern, const AdjArgs& a, int threads, size_t smem, int 
 
 template <typename KERN>
 hb_status adj_slots(KERN kern, int threads, size_t smem, int* slots) {
+  if (*slots) return HB_OK;
   int dev, sms = 0, per_sm = 0;
   HB_CUDA(cudaGetDevice(&dev));
   HB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -575,15 +577,15 @@ hb_status adj_one(const AdjCall& c) {
   if (d->np != S::NP || d->nfp != S::NFP)
     return fail(HB_ERR_UNSUPPORTED, "element sizes do not match the order");
   if (c.configure) {
-    hb_status st;
-    if ((st = adj_slots(adj_lift_kernel<MODEL, DIM, ORDER>, 128, S::ltotal, &op->adj_slots[0])) ||
-        (st = adj_slots(adj_element_kernel<MODEL, DIM, ORDER, false>, S::THREADS, S::total,
-                        &op->adj_slots[1])))
-      return st;
-    if (CW && (st = adj_slots(adj_element_kernel<MODEL, DIM, ORDER, CW>, SC::THREADS, SC::total,
-                              &op->adj_slots[2])))
-      return st;
-    return adj_fragments<MODEL, DIM, ORDER>(op);
+    hb_status st = adj_slots(adj_lift_kernel<MODEL, DIM, ORDER>, 128, S::ltotal,
+                             &op->adj_slots[0]);
+    if (st) return st;
+    st = c.want_c ? adj_slots(adj_element_kernel<MODEL, DIM, ORDER, CW>, SC::THREADS, SC::total,
+                              &op->adj_slots[2])
+                  : adj_slots(adj_element_kernel<MODEL, DIM, ORDER, false>, S::THREADS, S::total,
+                              &op->adj_slots[1]);
+    if (st || op->adjfrag) return st;
+    return adj_fragments<MODEL, DIM, ORDER>(op, c.stream);
   }
   const bool wc = c.a.c_bar != nullptr;
   AdjArgs a = c.a;
@@ -592,7 +594,7 @@ hb_status adj_one(const AdjCall& c) {
   a.lfrag = reinterpret_cast<const double2*>(op->adjfrag);
   a.afrag = a.lfrag + (size_t)S::LW * S::LSTEPS * S::LMW * 32;
   a.vfrag = a.afrag + (size_t)S::STEPS * S::MT * 32;
-  a.nlist = reinterpret_cast<const uint8_t*>(a.vfrag + (size_t)S::STEPS * S::MT * 32);
+  a.nlist = reinterpret_cast<const uint8_t*>(a.vfrag + (CW ? (size_t)S::STEPS * S::MT * 32 : 0));
   a.geo = d->geo;
   a.conn = op->conn;
   a.fmask = d->fmask;

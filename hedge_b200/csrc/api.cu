@@ -170,6 +170,7 @@ hb_status hb_discr_create(const hb_discr_desc* desc, hb_discr** out) {
       h[nd + (size_t)k * np + i] = desc->lift[(size_t)i * nf * nfp + k];
   std::memcpy(h + nd + nl, desc->geometry, sizeof(double) * ng);
   d->unit_nodes.assign(desc->unit_nodes, desc->unit_nodes + (size_t)np * dim);
+  d->fmask_host.assign(desc->fmask, desc->fmask + (size_t)nf * nfp);
   hb_status st;
   if ((st = upload(&d->dmats_t, h, nd)) || (st = upload(&d->lift_t, h + nd, nl)) ||
       (st = upload(&d->geo, h + nd + nl, ng)) ||
@@ -539,7 +540,7 @@ hb_status hb_adjoint_stage(hb_op* handle, double a, double b, double dt, const d
   if (st) return st;
   DeviceGuard g(op->d->device);
   if (!g.ok) return fail(HB_ERR_CUDA, "cannot select the CUDA device");
-  if (!adjoint_f64_ready(op, reinterpret_cast<cudaStream_t>(stream)))
+  if (!adjoint_f64_ready(op, c_bar != nullptr, reinterpret_cast<cudaStream_t>(stream)))
     return fail(HB_ERR_UNSUPPORTED, "adjoint stage: orders 1 to 7, and not as an operator's first "
                                     "adjoint under stream capture (compose it from "
                                     "hb_rhs_adjoint)");

@@ -2,13 +2,12 @@
 #pragma once
 
 #include <cuda_runtime.h>
-#include <atomic>
 #include <cstdint>
-#include <mutex>
 #include <string>
 #include <vector>
 
 #include "../../include/hedge_b200.h"
+#include "prepared.h"
 
 namespace hb {
 
@@ -77,6 +76,7 @@ struct Discr {
   // host copies kept for split-operator construction
   std::string host_blob;
   std::vector<double> unit_nodes;   // [np][dim]
+  std::vector<int> fmask_host;
 };
 
 struct Op {
@@ -101,10 +101,9 @@ struct Op {
   double* afrag = nullptr;
   int f64_slots[2] = {0, 0};   // CTAs resident on the GPU: fixed, variable material
   // the adjoint of an operator of order 1 to 7: fragments and resident CTAs
-  // (lift pass, element pass without and with the c gradient), made on its
-  // first adjoint call
-  std::mutex adj_mutex;
-  std::atomic<int> adj_state{0};   // 1: ready, 2: not built for this operator
+  // (lift pass, element pass without and with the c gradient), made on the
+  // first call without (variant 0) or with (1) the c gradient
+  Prepared adj;
   double* adjfrag = nullptr;
   int adj_slots[3] = {0, 0, 0};
   // split-precision operator planes (BF16X3)
@@ -134,9 +133,9 @@ hb_status launch_adjoint(Op* op, const double* q, const double* lam, double* q_b
 
 // the same on the FP64 tensor cores (adjoint_fp64.cu), operators of order 1 to
 // 7, and one stage of the reversed LSRK recurrences around it, in place
-// ready: prepares the operator on its first call, except under stream capture
-// (it allocates); false where the CUDA-core adjoint has to serve
-bool adjoint_f64_ready(Op* op, cudaStream_t s);
+// ready: prepares the operator on its first call of a variant, except under
+// stream capture (it allocates); false where the CUDA-core adjoint has to serve
+bool adjoint_f64_ready(Op* op, bool want_c, cudaStream_t s);
 hb_status launch_adjoint_f64(Op* op, const double* q, const double* lam, double* q_bar,
                              double* c_bar, const double* coeff, double* work, cudaStream_t s);
 hb_status launch_adjoint_stage(Op* op, double ra, double rb, double dt, const double* q,

@@ -267,7 +267,8 @@ hb_status hb_rhs_adjoint(hb_op* op, const double* q, const double* lam, double* 
  *   c_bar <- c_bar + dt (dR/dc)^T lam  (unless NULL);   lam <- a lam
  * with lam, lq [F][K*Np], c_bar [K*Np] and the other arguments as in
  * hb_rhs_adjoint; none of lam, lq and q may overlap.  Orders 1 to 7, and not
- * as an operator's first adjoint call under stream capture, else
+ * as an operator's first adjoint call (of those with, of those without c_bar)
+ * under stream capture, else
  * HB_ERR_UNSUPPORTED (compose the stage from hb_rhs_adjoint). */
 hb_status hb_adjoint_stage(hb_op* op, double a, double b, double dt, const double* q,
                            double* lam, double* lq, double* c_bar, const double* coeff,
