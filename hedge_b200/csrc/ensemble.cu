@@ -97,7 +97,7 @@ __device__ __forceinline__ void ens_tile(const EnsInst& I, const EnsTile& T, con
   constexpr int F = Traits<MODEL, DIM>::F;
   constexpr int NA = F;   // no coefficient field in the batch models
   constexpr int NF = DIM + 1;
-  constexpr int UNROLL = ORDER ? 4 : 1;
+  constexpr int UNROLL = 4;
   constexpr int CNP = DIM == 2 ? (ORDER + 1) * (ORDER + 2) / 2
                                : (ORDER + 1) * (ORDER + 2) * (ORDER + 3) / 6;
   constexpr int CNFP = DIM == 2 ? ORDER + 1 : (ORDER + 1) * (ORDER + 2) / 2;
@@ -233,12 +233,14 @@ __device__ __forceinline__ void ens_tile(const EnsInst& I, const EnsTile& T, con
 // 3D, whose nodes hold more values, 6 (40 registers).  Measured on 20 2D members
 // of order 3 to 6, K = 500 to 20000, per LSRK4 step: 560 us with run-time
 // element sizes at 6 CTAs; compile-time sizes 482 us; the residual requested
-// ahead of the lift 465 us; 8 CTAs 451 us.
-template <int DIM>
-__global__ void __launch_bounds__(ENS_THREADS, DIM == 2 ? 8 : 6) ens_kernel(const EnsInst* __restrict__ insts,
-                                                             const EnsTile* __restrict__ tiles,
-                                                             int ntiles, EnsLayout L, double ra,
-                                                             double rb, int src, int* err) {
+// ahead of the lift 465 us; 8 CTAs 451 us.  A batch that is mostly beyond order 7
+// takes the build with run-time sizes only (ANY) and 6 CTAs: as one more case of
+// the switch at 8 CTAs, 24 members of order 8 took 2.26 ms a step against 1.94
+// ms, of order 9 3.06 against 2.67 ms.
+template <int DIM, bool ANY>
+__global__ void __launch_bounds__(ENS_THREADS, DIM == 2 && !ANY ? 8 : 6)
+    ens_kernel(const EnsInst* __restrict__ insts, const EnsTile* __restrict__ tiles, int ntiles,
+               EnsLayout L, double ra, double rb, int src, int* err) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x;
   const float* cached = nullptr;   // operators resident in shared memory
@@ -259,23 +261,26 @@ __global__ void __launch_bounds__(ENS_THREADS, DIM == 2 ? 8 : 6) ens_kernel(cons
       cached = I.dmats_t;
     }
     const bool adv = I.model == HB_MODEL_ADVECTION;
-#define HB_ENS_ORDER(O)                                                                  \
-  case O:                                                                                \
-    if (adv)                                                                             \
-      ens_tile<HB_MODEL_ADVECTION, DIM, O>(I, T, L, smem, ra, rb, src, err);             \
-    else                                                                                 \
-      ens_tile<HB_MODEL_WAVE, DIM, O>(I, T, L, smem, ra, rb, src, err);                  \
-    break;
-    switch (I.order) {
-      HB_ENS_ORDER(1) HB_ENS_ORDER(2) HB_ENS_ORDER(3) HB_ENS_ORDER(4)
-      HB_ENS_ORDER(5) HB_ENS_ORDER(6) HB_ENS_ORDER(7)
-      default:
-        if (adv)
-          ens_tile<HB_MODEL_ADVECTION, DIM, 0>(I, T, L, smem, ra, rb, src, err);
-        else
-          ens_tile<HB_MODEL_WAVE, DIM, 0>(I, T, L, smem, ra, rb, src, err);
+#define HB_ENS_TILE(O)                                                                   \
+  if (adv)                                                                               \
+    ens_tile<HB_MODEL_ADVECTION, DIM, O>(I, T, L, smem, ra, rb, src, err);               \
+  else                                                                                   \
+    ens_tile<HB_MODEL_WAVE, DIM, O>(I, T, L, smem, ra, rb, src, err);
+    if constexpr (ANY) {
+      HB_ENS_TILE(0)
+    } else {
+      switch (I.order) {
+        case 1: HB_ENS_TILE(1) break;
+        case 2: HB_ENS_TILE(2) break;
+        case 3: HB_ENS_TILE(3) break;
+        case 4: HB_ENS_TILE(4) break;
+        case 5: HB_ENS_TILE(5) break;
+        case 6: HB_ENS_TILE(6) break;
+        case 7: HB_ENS_TILE(7) break;
+        default: HB_ENS_TILE(0)
+      }
     }
-#undef HB_ENS_ORDER
+#undef HB_ENS_TILE
   }
 }
 
@@ -286,7 +291,8 @@ struct Batch {
   EnsInst* d_insts = nullptr;
   EnsTile* d_tiles = nullptr;
   int* err = nullptr;
-  int ntiles = 0, grid = 0, dim = 2;
+  int ntiles = 0, grid = 0;
+  decltype(&ens_kernel<2, false>) kern = nullptr;
   EnsLayout L{};
   int64_t dofs = 0;
 };
@@ -378,8 +384,12 @@ hb_status batch_create(const hb_batch_member* m, int32_t n, Batch** out) {
           cudaSuccess)
     return bail(fail(HB_ERR_CUDA, "batch: device query"));
   if (B->L.total > (size_t)max_optin) return bail(fail(HB_ERR_UNSUPPORTED, "batch: tiles too large"));
-  auto kern = dim == 2 ? ens_kernel<2> : ens_kernel<3>;
-  B->dim = dim;
+  int64_t any = 0;   // DOFs of the members with run-time sizes
+  for (const EnsInst& I : insts) any += I.order ? 0 : I.K * I.np * I.F;
+  const bool built = 2 * any <= dofs;
+  B->kern = dim == 2 ? (built ? ens_kernel<2, false> : ens_kernel<2, true>)
+                     : (built ? ens_kernel<3, false> : ens_kernel<3, true>);
+  auto kern = B->kern;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)B->L.total) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ENS_THREADS, B->L.total) !=
@@ -411,9 +421,8 @@ void batch_destroy(Batch* B) {
 hb_status batch_stage(Batch* B, double a, double b, int parity, cudaStream_t s) {
   DeviceGuard g(B->device);
   if (!g.ok) return fail(HB_ERR_CUDA, "cannot select the CUDA device");
-  auto kern = B->dim == 2 ? ens_kernel<2> : ens_kernel<3>;
-  kern<<<B->grid, ENS_THREADS, B->L.total, s>>>(B->d_insts, B->d_tiles, B->ntiles, B->L, a, b,
-                                                parity & 1, B->err);
+  B->kern<<<B->grid, ENS_THREADS, B->L.total, s>>>(B->d_insts, B->d_tiles, B->ntiles, B->L, a, b,
+                                                   parity & 1, B->err);
   HB_CUDA(cudaGetLastError());
   return HB_OK;
 }
