@@ -116,8 +116,6 @@ static hb_status upload_quadrature(Op* op, const hb_quad_desc* qd) {
       h[nI + nB + nF + (size_t)p * np + i] = qd->face_lift[(size_t)i * nf * nqf + p];
   for (double x : h)
     if (!std::isfinite(x)) return fail(HB_ERR_INVALID_ARGUMENT, "non-finite quadrature matrix");
-  op->nq = nq;
-  op->nqf = nqf;
   // FP64 matrices for both precisions (the FP32 path computes in FP64)
   return upload(&op->quad64, h.data(), h.size());
 }
@@ -303,7 +301,9 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
     // buffer of the element maxima the LF flux reads
     if (cudaMalloc(&op->elmax, sizeof(double) * d->K) != cudaSuccess)
       return bail(fail(HB_ERR_CUDA, "cannot allocate the element maxima"));
-    st = prepare_quad_f64(op, qd);
+    op->nq = qd->nq;
+    op->nqf = qd->nqf;
+    st = quad_on_cores(op) ? HB_ERR_UNSUPPORTED : prepare_quad_f64(op, qd);
     if (st == HB_ERR_UNSUPPORTED) {
       st = upload_quadrature(op, qd);
       if (!st) st = prepare_quad(op);

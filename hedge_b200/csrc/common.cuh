@@ -163,6 +163,7 @@ hb_status prepare_f64(Op* op);
 
 // quadrature kernel (rhs_quad.cu); vel = the velocity field [dim][K*Np]
 hb_status prepare_quad(Op* op);
+bool quad_on_cores(Op* op);   // whether it is the faster one
 // its FP64 tensor-core form (quad_fp64.cu), for the element sizes built
 hb_status prepare_quad_f64(Op* op, const hb_quad_desc* qd);
 hb_status launch_quad_f64(Op* op, int mode, double ra, double rb, double dt, const void* q_in,

@@ -350,8 +350,6 @@ hb_status prepare_quad_f64(Op* op, const hb_quad_desc* qd) {
     }
   for (double x : h)
     if (!std::isfinite(x)) return fail(HB_ERR_INVALID_ARGUMENT, "non-finite quadrature matrix");
-  op->nq = nq;
-  op->nqf = nqf;
   if (cudaMalloc(&op->quadfrag, sizeof(double) * h.size()) != cudaSuccess ||
       cudaMemcpy(op->quadfrag, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice) !=
           cudaSuccess)
@@ -359,6 +357,7 @@ hb_status prepare_quad_f64(Op* op, const hb_quad_desc* qd) {
   const int per_cta = 8 * (QUAD_THREADS / 32);
   op->elems_per_block = per_cta;
   op->threads = QUAD_THREADS;
+  op->blocks_per_sm = 0;
   op->smem = 0;
   op->ops_in_smem = 0;
   op->grid = (int)((d->K + per_cta - 1) / per_cta);

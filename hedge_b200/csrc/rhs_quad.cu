@@ -462,6 +462,35 @@ hb_status prepare_quad(Op* op) {
                                        nullptr, 0, true);
 }
 
+// The element sizes and meshes that stay on this file's kernel, with the
+// operator's sizes and point counts (stage times here -> quad_fp64.cu):
+//   meshes of one round of this kernel's CTAs, where a batch's chain counts and
+//   the tensor-core form has one warp's: 2D order 6 (K <= 1250 15.8 -> 17.1 us; K = 1568
+//   18.8 -> 17.3), 3D orders 3 and 4 with the matrices in shared memory (order 3, degree
+//   9: K <= 1296 25.1 -> 28.7, K = 2058 44.8 -> 29.1; order 4, degree 9: K <= 750 25.2 -> 34.6,
+//   K = 1296 43.7 -> 34.9) and 3D order 5 with few points (degree 11: K <= 750 53 -> 59);
+//   two rounds at 2D order 7, whose tensor-core form runs at 250 registers
+//   (degree 21: K <= 800 20 -> 41, K = 2048 34 -> 41, K = 3200 60 -> 42);
+//   2D order 1 beyond one round of the tensor-core form (K = 20000 9.5 -> 7.9, K =
+//   24200 9.5 -> 12.1, K = 80000 17 -> 24), and 3D order 2 on a single warp (K = 6 11.3 ->
+//   13.7, K = 48 19 -> 14.5).
+bool quad_on_cores(Op* op) {
+  const Discr* d = op->d;
+  const int np = d->np;
+  if (d->dim == 2 && np == 3) return d->K > 20480;
+  if (d->dim == 3 && np == 10) return d->K <= 8;
+  int rounds = 0;
+  if (d->dim == 2) rounds = np == 28 ? 1 : np == 36 ? 2 : 0;
+  if (d->dim == 3) rounds = np == 20 || np == 35 || (np == 56 && op->nq <= 128) ? 1 : 0;
+  if (!rounds || prepare_quad(op) != HB_OK) return false;
+  if (d->dim == 3 && np != 56 && !op->ops_in_smem) return false;
+  int dev, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return false;
+  return d->K <= (int64_t)op->elems_per_block * op->blocks_per_sm * sms * rounds;
+}
+
 hb_status launch_quad(Op* op, int mode, double ra, double rb, double dt, const void* q_in,
                       void* q_out, void* res, const double* vel, const double* bdry,
                       cudaStream_t s) {
