@@ -1616,9 +1616,10 @@ struct ShapeS {
                                F * SQS * 4 <= (int)(2 * bAq);
 };
 
-// 32 bytes from a 32-byte boundary
+// 32 bytes from a 32-byte boundary.  Volatile: the previous launch wrote them,
+// so the load stays behind griddepcontrol.wait
 __device__ __forceinline__ void ldg4(const double* p, double* v) {
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
       : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
       : "l"(p));
 }
