@@ -383,15 +383,15 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER>::THREADS,
       }
 #pragma unroll
       for (int f = 0; f < F; ++f) {
-        we[f] = __ldg(a.work + ((el0 + e) * NFPT + p) * F + f);
-        wn[f] = nb >= 0 ? __ldg(a.work + (nb * NFPT + pn) * F + f) : 0.0;
-        if constexpr (WC) qn[f] = nb >= 0 ? __ldg(a.q + f * Knp + nb * NP + nn) : 0.0;
+        we[f] = a.work[((el0 + e) * NFPT + p) * F + f];
+        wn[f] = nb >= 0 ? a.work[(nb * NFPT + pn) * F + f] : 0.0;
+        if constexpr (WC) qn[f] = nb >= 0 ? a.q[f * Knp + nb * NP + nn] : 0.0;
       }
 #pragma unroll
       for (int d = 0; d < DIM; ++d)
         nnb[d] = nb >= 0 ? __ldg(a.geo + nb * G + DIM * DIM + (cn.y & 3) * (DIM + 1) + d) : 0.0;
       const double cm = C ? sc[e * NP + lnode] : 0.0;
-      const double cp = (C && nb >= 0) ? __ldg(a.coeff + nb * NP + nn) : cm;
+      const double cp = (C && nb >= 0) ? a.coeff[nb * NP + nn] : cm;
       double* w = sw + e * CF * NFPT + p;
 #pragma unroll
       for (int g = 0; g < F; ++g) {

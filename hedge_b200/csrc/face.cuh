@@ -57,12 +57,12 @@ __device__ __forceinline__ void face_load(const FaceArgs<S>& a, const int2 cn, i
     return;
   }
   const int64_t gi = (int64_t)cn.x * np + nbr_node[(perm * nf + nface) * nfp + k];
-  if constexpr (C != 0) x.u[0] = __ldg(a.coeff + gi);
+  if constexpr (C != 0) x.u[0] = a.coeff[gi];
 #pragma unroll
-  for (int f = 0; f < F; ++f) x.u[C + f] = (double)__ldg(a.q + f * Knp + gi);
+  for (int f = 0; f < F; ++f) x.u[C + f] = (double)a.q[f * Knp + gi];
   if constexpr (VM) {
-    x.eps = __ldg(a.coeff + gi);
-    x.mu = __ldg(a.coeff + Knp + gi);
+    x.eps = a.coeff[gi];
+    x.mu = a.coeff[Knp + gi];
   }
 }
 
@@ -93,7 +93,7 @@ __device__ __forceinline__ bool face_flux(const FaceArgs<S>& a, const ModelParam
         atomicCAS(a.err, 0, a.bdry == nullptr ? DEV_MISSING_INPUT : DEV_BAD_BDRY_INDEX);
         have = false;
       } else {
-        given = __ldg(a.bdry + bi);
+        given = a.bdry[bi];
       }
     }
     if (have) {
@@ -115,7 +115,7 @@ __device__ __forceinline__ bool face_flux(const FaceArgs<S>& a, const ModelParam
           have = false;
         } else {
 #pragma unroll
-          for (int f = 0; f < F; ++f) x.u[f] = -__ldg(a.bdry + f * a.n_given + bi);
+          for (int f = 0; f < F; ++f) x.u[f] = -a.bdry[f * a.n_given + bi];
         }
       }
     }

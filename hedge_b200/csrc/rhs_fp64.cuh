@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(F64Shape<MODEL, DIM, ORDER, sizeof(IO)>::THREA
 #pragma unroll
           for (int f = 0; f < F; ++f) {
             rv[u][f] = a.res[f * Knp + base + u * THREADS];
-            qv[u][f] = __ldg(a.face.q + f * Knp + base + u * THREADS);
+            qv[u][f] = a.face.q[f * Knp + base + u * THREADS];
           }
         }
     }
