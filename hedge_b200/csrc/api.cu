@@ -321,6 +321,7 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
     }
     if (st == HB_ERR_UNSUPPORTED) {
       free_split(op);
+      op->wide = model == HB_MODEL_ADVECTION && d->order <= 2;
       st = prepare_simt(op);
     }
   } else {

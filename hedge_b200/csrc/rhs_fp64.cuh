@@ -521,6 +521,20 @@ inline bool f64_fp32_mesh(int model, int dim, int order, int64_t k) {
   return !even || k <= 16384;
 }
 
+// Advection of low order on larger meshes stays on the CUDA cores: one field
+// makes tiles of many small elements, whose point phases outweigh the product
+// (stage times, CUDA cores -> here): 2D order 2, K = 24200 7.0 -> 7.7 us (K = 16200 6.5
+// -> 6.6); 3D order 1, K = 24576 7.6 -> 8.0, K = 34992 8.5 -> 9.9 (FP32 states K = 13182 7.1 ->
+// 8.0); 3D order 2, K = 1296 6.8 -> 7.1, K = 10368 8.7 -> 10.4, K = 48000 23 -> 29.  FP32
+// states keep their FP64 arithmetic there; of 3D order 3 they go to the split
+// planes (K = 16464 16.3 -> 16.8, K = 48000 35 -> 46).
+inline bool f64_mesh(int model, int dim, int order, bool fp32, int64_t k) {
+  if (model != HB_MODEL_ADVECTION) return true;
+  if (dim == 2) return order != 2 || k <= 16384;
+  return order == 1 ? k <= (fp32 ? 12288 : 16384) : order == 2 ? k <= 1024
+                    : order != 3 || !fp32 || k <= 16384;
+}
+
 // Maxwell: the variable-material kernel where the call gives the material
 template <int MODEL, int DIM, int ORDER, typename IO>
 hb_status f64_material(const F64Call& c) {
@@ -535,7 +549,10 @@ hb_status f64_material(const F64Call& c) {
 
 template <int MODEL, int DIM, int ORDER>
 hb_status f64_order(const F64Call& c) {
-  if (c.op->precision == HB_PREC_FP32) {
+  const bool fp32 = c.op->precision == HB_PREC_FP32;
+  if (c.configure && !f64_mesh(MODEL, DIM, ORDER, fp32, c.op->d->K))
+    return fail(HB_ERR_UNSUPPORTED, "FP64 tensor-core kernel: slower on this mesh");
+  if (fp32) {
     // FP32 states: the elements and meshes that are faster here
     if constexpr (f64_fp32_state(MODEL, DIM, ORDER)) {
       if (!c.configure || f64_fp32_mesh(MODEL, DIM, ORDER, c.op->d->K))

@@ -444,7 +444,25 @@ static hb_status dispatch(Op* op, int mode, double ra, double rb, double dt,
   return fail(HB_ERR_UNSUPPORTED, "model/dimension combination not built");
 }
 
+// FP32 advection of low order keeps the FP64 arithmetic that it has on the
+// tensor cores (rhs_fp64.cuh, f64_mesh)
+static hb_status dispatch_wide(Op* op, int mode, double ra, double rb, double dt,
+                               const void* q_in, void* q_out, void* res, const double* coeff,
+                               const double* bdry, const double* source, int64_t e0, int64_t e1,
+                               cudaStream_t s, bool configure) {
+  return op->d->dim == 2
+             ? launch_one<HB_MODEL_ADVECTION, 2, double, float>(op, mode, ra, rb, dt, q_in, q_out,
+                                                                res, coeff, bdry, source, e0, e1,
+                                                                s, configure)
+             : launch_one<HB_MODEL_ADVECTION, 3, double, float>(op, mode, ra, rb, dt, q_in, q_out,
+                                                                res, coeff, bdry, source, e0, e1,
+                                                                s, configure);
+}
+
 hb_status prepare_simt(Op* op) {
+  if (op->wide)
+    return dispatch_wide(op, 0, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0,
+                         op->d->K, 0, true);
   if (op->precision == HB_PREC_FP32)
     return dispatch<float, float>(op, 0, 0, 0, 0, nullptr, nullptr, nullptr,
                                   nullptr, nullptr, nullptr, 0, op->d->K, 0, true);
@@ -456,6 +474,9 @@ hb_status launch_simt(Op* op, int mode, double ra, double rb, double dt,
                       const void* q_in, void* q_out, void* res,
                       const double* coeff, const double* bdry,
                       const double* source, int64_t e0, int64_t e1, cudaStream_t s) {
+  if (op->wide)
+    return dispatch_wide(op, mode, ra, rb, dt, q_in, q_out, res, coeff, bdry, source, e0, e1, s,
+                         false);
   if (op->precision == HB_PREC_FP32)
     return dispatch<float, float>(op, mode, ra, rb, dt, q_in, q_out, res, coeff,
                                   bdry, source, e0, e1, s, false);
