@@ -269,6 +269,7 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
   Op* op = new (std::nothrow) Op();
   if (!op) return fail(HB_ERR_INVALID_ARGUMENT, "out of host memory");
   op->d = d;
+  op->device = d->device;
   op->model = model;
   op->F = F;
   // FP32_SIMT is the FP32 path kept on the CUDA cores
@@ -336,7 +337,7 @@ hb_status hb_op_create(hb_discr* discr, const hb_op_desc* desc, hb_op** out) {
 hb_status hb_op_destroy(hb_op* handle) {
   if (!handle) return HB_OK;
   Op* op = reinterpret_cast<Op*>(handle);
-  DeviceGuard g(op->d->device);
+  DeviceGuard g(op->device);
   cudaFree(op->conn);
   cudaFree(op->err_flag);
   cudaFree(op->quad64); cudaFree(op->quadfrag); cudaFree(op->elmax); cudaFree(op->afrag); cudaFree(op->adjfrag);
@@ -363,11 +364,11 @@ static hb_status check_inputs(Op* op, const void* q_in, const void* q_out,
   const bool fixed = op->split || (op->model == HB_MODEL_MAXWELL && op->afrag &&
                                    op->precision == HB_PREC_FP32 && op->d->order >= 3);
   if (maxwell && coeff && fixed)
-    return fail(HB_ERR_UNSUPPORTED, "Maxwell with variable material: CUDA-core kernels only "
-                                    "(HB_PREC_FP64, HB_PREC_FP32_SIMT)");
+    return fail(HB_ERR_UNSUPPORTED, "Maxwell with variable material: HB_PREC_FP64 or "
+                                    "HB_PREC_FP32_SIMT only");
   if (maxwell && bdry && fixed)
-    return fail(HB_ERR_UNSUPPORTED, "Maxwell incident data: CUDA-core kernels only "
-                                    "(HB_PREC_FP64, HB_PREC_FP32_SIMT)");
+    return fail(HB_ERR_UNSUPPORTED, "Maxwell incident data: HB_PREC_FP64 or HB_PREC_FP32_SIMT "
+                                    "only");
   return HB_OK;
 }
 

@@ -81,6 +81,7 @@ struct Discr {
 
 struct Op {
   Discr* d;
+  int device;                // d's, for hb_op_destroy, which may come after d's
   int model, F, precision;   // precision: HB_PREC_FP64 .. HB_PREC_FP16X3 (FP32_SIMT is stored as FP32)
   int split = 0;             // 1: the tensor-core kernels (launch_split), else CUDA cores
   int wide = 0;              // CUDA cores: FP32 states in FP64 arithmetic

@@ -454,7 +454,7 @@ class CompiledOperator:
         if self.var_material or self.incident_data:
             if prec in (_native.PREC_BF16X3, _native.PREC_FP16X3):
                 raise NotImplementedError(
-                    "Maxwell with %s: fp64 or fp32 (CUDA-core kernels)"
+                    "Maxwell with %s: fp64 or fp32"
                     % ("variable material" if self.var_material else "incident data"))
             if prec == _native.PREC_FP32:
                 prec = _native.PREC_FP32_SIMT
