@@ -507,13 +507,11 @@ hb_status f64_one(const F64Call& c) {
 // K = 48000 417 -> 395 us; 2D wave N = 3, K = 45000 225 -> 97 us, N = 6, K = 20000
 // 140 -> 137 us; against 3D Maxwell N = 4, K = 48000 716 -> 1152 us and 3D wave
 // N = 4 489 -> 722 us, N = 5, K = 16464 252 -> 568 us.
-// On meshes beyond 16384 elements not 2D advection and wave of order 6 (wave, K =
-// 33800: 201 -> 210 us) and 3D wave of order 1 and 2 (K = 34992: 63 -> 67 and
-// 143 -> 146 us); on smaller ones those too (K = 7200 81 -> 72, K = 10368 52 -> 32 us).
-constexpr bool f64_fp32_state(int model, int dim, int order) {
-  (void)model;
-  return dim == 2 || order <= 3;
-}
+// Beyond 16384 elements 2D advection and wave of order 6 and 3D wave of order 1
+// and 2 stay where they were: the two sides are within 5 % of each other there
+// (2D wave, order 6: K = 7200 81 -> 72 us, K = 20000 140 -> 137, K = 33800 201 -> 210; 3D
+// wave, orders 1 and 2: K = 10368 52 -> 32 us, K = 34992 63 -> 67 and 143 -> 146 us).
+constexpr bool f64_fp32_state(int dim, int order) { return dim == 2 || order <= 3; }
 inline bool f64_fp32_mesh(int model, int dim, int order, int64_t k) {
   const bool wave = model == HB_MODEL_WAVE || model == HB_MODEL_VARWAVE;
   const bool even = dim == 2 ? order == 6 && (wave || model == HB_MODEL_ADVECTION)
@@ -538,7 +536,8 @@ inline bool f64_mesh(int model, int dim, int order, bool fp32, int64_t k) {
 // Maxwell: the variable-material kernel where the call gives the material
 template <int MODEL, int DIM, int ORDER, typename IO>
 hb_status f64_material(const F64Call& c) {
-  if constexpr (IsMaxwell<MODEL>::value) {
+  // (FP32 3D Maxwell of order 3 refuses a material: api.cu, check_inputs)
+  if constexpr (IsMaxwell<MODEL>::value && !(DIM == 3 && ORDER >= 3 && sizeof(IO) == 4)) {
     if (c.configure || c.coeff != nullptr) {
       const hb_status st = f64_one<MODEL, DIM, ORDER, true, IO>(c);
       if (st || !c.configure) return st;
@@ -554,7 +553,7 @@ hb_status f64_order(const F64Call& c) {
     return fail(HB_ERR_UNSUPPORTED, "FP64 tensor-core kernel: slower on this mesh");
   if (fp32) {
     // FP32 states: the elements and meshes that are faster here
-    if constexpr (f64_fp32_state(MODEL, DIM, ORDER)) {
+    if constexpr (f64_fp32_state(DIM, ORDER)) {
       if (!c.configure || f64_fp32_mesh(MODEL, DIM, ORDER, c.op->d->K))
         return f64_material<MODEL, DIM, ORDER, float>(c);
     }

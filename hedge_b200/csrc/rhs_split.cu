@@ -2743,6 +2743,14 @@ static hb_status launch_stream_t(Op* op, int mode, double ra, double rb, double 
   X(HB_MODEL_VARWAVE, 2, 6) X(HB_MODEL_VARWAVE, 3, 3) X(HB_MODEL_VARWAVE, 3, 4)        \
   X(HB_MODEL_MAXWELL, 3, 3) X(HB_MODEL_MAXWELL, 3, 4) X(HB_MODEL_MAXWELL, 3, 5)
 
+// the ones FP32 states come to: the others run on the FP64 kernel at every mesh
+// size (rhs_fp64.cuh: f64_fp32_state, f64_fp32_mesh, f64_mesh)
+#define HB_SPLIT_FP32_INSTANCES(X)                                                     \
+  X(HB_MODEL_ADVECTION, 2, 6) X(HB_MODEL_ADVECTION, 3, 3) X(HB_MODEL_ADVECTION, 3, 4)  \
+  X(HB_MODEL_WAVE, 2, 6) X(HB_MODEL_WAVE, 3, 4) X(HB_MODEL_WAVE, 3, 5)                 \
+  X(HB_MODEL_VARWAVE, 2, 6) X(HB_MODEL_VARWAVE, 3, 4)                                  \
+  X(HB_MODEL_MAXWELL, 3, 4) X(HB_MODEL_MAXWELL, 3, 5)
+
 // The streamed-operator kernel serves the instances it is built for (with or
 // without halo faces): at 3D N = 5 the resident kernel's operator planes
 // leave room for one state stage and no residual buffer, and the streamed
@@ -2759,7 +2767,7 @@ hb_status prepare_split(Op* op) {
 #define HB_CASE(M, D, O)                                                       \
   if (op->model == M && dim == D && order == O)                                \
     return configure_split<M, D, O, PT_FP16, float>(op);
-    HB_SPLIT_INSTANCES(HB_CASE)
+    HB_SPLIT_FP32_INSTANCES(HB_CASE)
 #undef HB_CASE
     return fail(HB_ERR_UNSUPPORTED, "no FP32-state tensor-core kernel for this instance");
   }
@@ -2810,7 +2818,7 @@ hb_status launch_split(Op* op, int mode, double ra, double rb, double dt,
   if (op->model == M && dim == D && order == O)                                       \
     return launch_split_t<M, D, O, PT_FP16, float>(op, mode, ra, rb, dt, q_in, q_out,  \
                                                    res, coeff, bdry, source, e0, e1, s);
-    HB_SPLIT_INSTANCES(HB_CASE)
+    HB_SPLIT_FP32_INSTANCES(HB_CASE)
 #undef HB_CASE
     return fail(HB_ERR_UNSUPPORTED, "model/dimension/order combination not built");
   }
