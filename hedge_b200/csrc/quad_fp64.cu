@@ -15,8 +15,10 @@
 // in fragment order through L1, which they share on an SM.
 //
 // Bound: FP64 pipe (N = 5, 64 volume points: 294 MMAs per 8 elements, 40 us at
-// K = 80000) and L1 wavefronts of the scattered 8-byte gathers.  The element
-// sizes are run-time values except the number of 8-node tiles KS.
+// K = 80000) and L1 wavefronts of the scattered 8-byte gathers.  A stage at K =
+// 80000, N = 5: 219 -> 72 us, N = 3 66 -> 36, N = 7 1178 -> 249 (rhs_quad.cu -> here); the
+// sizes and meshes that stay there are in quad_on_cores.  The element sizes are
+// run-time values except the number of 8-node tiles KS.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -31,7 +33,7 @@ namespace {
 template <typename IO>
 struct QuadF64Args {
   int64_t K, n_given;
-  int np, nfp, nf, nperm, G, nq, nqf;
+  int np, nfp, nf, nperm, G, mode, flux_type;
   int nqt, nft;                 // tiles of 8 volume points, face points
   const double2* If;            // [nqt][KS][32]
   const double2* Pf;            // [dim][nqt][KS][32]
@@ -48,7 +50,6 @@ struct QuadF64Args {
   const double* bdry;
   const double* elmax;          // element maxima of |v|^2 (LF flux)
   double ra, rb, dt;
-  int mode, flux_type;
   int* err;
 };
 
@@ -113,8 +114,7 @@ __global__ void __launch_bounds__(QUAD_THREADS) quad_fp64_kernel(const QuadF64Ar
           double s = 0.0;
 #pragma unroll
           for (int x = 0; x < DIM; ++x) s += rx[r][x] * c[1 + x][h];
-          // (points beyond the last are 0 * w, not zero where w is not finite)
-          gr[h] = 8 * qt + 2 * t + h < a.nq ? c[0][h] * s : 0.0;
+          gr[h] = c[0][h] * s;
         }
 #pragma unroll
         for (int m = 0; m < KS; ++m) {
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(QUAD_THREADS) quad_fp64_kernel(const QuadF64Ar
           v = 0.5 * (nvm * cm[0][h] + nvp * cp[0][h]) - 0.5 * (cp[0][h] - cm[0][h]) * cmax;
         else
           v = navg > 0.0 ? nvm * cm[0][h] : nvp * cp[0][h];
-        fl[h] = none || 8 * pt + 2 * t + h >= a.nqf ? 0.0 : fscale * v;
+        fl[h] = none ? 0.0 : fscale * v;
       }
 #pragma unroll
       for (int m = 0; m < KS; ++m) {
@@ -272,8 +272,6 @@ hb_status quad_run(const QuadCall& c) {
   a.nf = d->nfaces;
   a.nperm = d->nperm;
   a.G = d->G;
-  a.nq = op->nq;
-  a.nqf = op->nqf;
   a.nqt = (op->nq + 7) / 8;
   a.nft = (op->nqf + 7) / 8;
   a.If = reinterpret_cast<const double2*>(op->quadfrag);
@@ -332,18 +330,25 @@ hb_status prepare_quad_f64(Op* op, const hb_quad_desc* qd) {
   double* P = I + nI;
   double* F = P + nP;
   double* L = F + nF;
+  // the points that pad a tile repeat the last one, against zeros in the
+  // projection and the lift: as 0 * w their values would not be zero where w is
+  // not finite, also where the flux of the points does not see that w
+  // (selecting zeros in the kernel instead: 72 -> 76 us a stage at N = 5, K = 80000)
+  for (int q = 0; q < 8 * nqt; ++q)
+    for (int j = 0; j < np; ++j)
+      I[at((size_t)(q / 8) * ks + j / 8, q % 8, j % 8)] =
+          qd->vol_interp[(size_t)std::min(q, nq - 1) * np + j];
   for (int q = 0; q < nq; ++q)
-    for (int j = 0; j < np; ++j) {
-      I[at((size_t)(q / 8) * ks + j / 8, q % 8, j % 8)] = qd->vol_interp[(size_t)q * np + j];
+    for (int j = 0; j < np; ++j)
       for (int r = 0; r < dim; ++r)
         P[at(((size_t)r * nqt + q / 8) * ks + j / 8, j % 8, q % 8)] =
             qd->vol_project[((size_t)r * np + j) * nq + q];
-    }
   for (int f = 0; f < nf; ++f)
-    for (int p = 0; p < nqf; ++p) {
+    for (int p = 0; p < 8 * nft; ++p) {
       for (int k = 0; k < nfp; ++k)
         F[at(((size_t)f * nft + p / 8) * kf + k / 8, p % 8, k % 8)] =
-            qd->face_interp[((size_t)f * nqf + p) * nfp + k];
+            qd->face_interp[((size_t)f * nqf + std::min(p, nqf - 1)) * nfp + k];
+      if (p >= nqf) continue;
       for (int i = 0; i < np; ++i)
         L[at(((size_t)f * nft + p / 8) * ks + i / 8, i % 8, p % 8)] =
             -qd->face_lift[((size_t)i * nf + f) * nqf + p];
