@@ -190,12 +190,13 @@ class ReceiverTraces:
                     cc = cc if ctx.has_c else None
                     comp, rec, dt = ctx.comp, ctx.receivers, ctx.dt
                     want_c = ctx.has_c and ctx.needs_input_grad[1]
-                    # lq is updated in place: an FP64 copy of its own, whatever
-                    # the receivers return
+                    # lq is updated in place: FP64 and its own, whatever a
+                    # user's receivers return (Receivers make a new tensor)
                     q_last = ctx.checkpoints[0]
                     lq = rec.transpose(g[ctx.nsteps], q_last)
-                    lq = torch.empty(q_last.shape, dtype=torch.float64,
-                                     device=q_last.device).copy_(lq)
+                    if type(rec) is not Receivers or lq.dtype != torch.float64:
+                        lq = torch.empty(q_last.shape, dtype=torch.float64,
+                                         device=q_last.device).copy_(lq)
                     c_bar = torch.zeros_like(cc) if want_c else None
                     starts = sorted(ctx.checkpoints)
                     ends = starts[1:] + [ctx.nsteps]
@@ -215,9 +216,8 @@ class ReceiverTraces:
                         for n in range(s1 - 1, s0 - 1, -1):
                             keep = stages[n - s0]
                             lres = torch.zeros_like(lq)
-                            for s in range(4, -1, -1):
-                                comp.adjoint_stage(RK4A[s], RK4B[s], dt, lres, lq,
-                                                   q=keep[s], coeff=cc, c_bar=c_bar)
+                            comp.adjoint_step(RK4A, RK4B, dt, lres, lq, keep, coeff=cc,
+                                              c_bar=c_bar)
                             lq = (lq + rec.transpose(g[n], lq)).contiguous()
                     q0_bar = lq.reshape(ctx.checkpoints[0].shape)
                     return q0_bar, c_bar, None, None, None, None, None, None

@@ -707,17 +707,19 @@ class CompiledOperator:
         is given, source hold for all of them."""
         n = len(a)
         if len(b) != n or len(bufs) != n + 1 or \
-                any(getattr(x, "_type_", None) is not C.c_double for x in (a, b)):
+                getattr(a, "_type_", None) is not C.c_double or \
+                getattr(b, "_type_", None) is not C.c_double:
             raise ValueError("%d stages need %d coefficients a and b (ctypes doubles) and %d "
                              "buffers" % (n, n, n + 1))
         keep, bptr = self._bdry_ptr(bc_in)
         if source_stride:
-            rows = (self._n_e or 1) * len(self.discr)
+            d = self.discr
+            rows = (self._n_e or 1) * len(d)
             if self.var_material:
                 raise ValueError("variable material: one source for all stages")
-            if source_stride < 0 or source.dtype != _torch().float64 or \
-                    not source.is_contiguous() or source.device != self.discr.device or \
-                    source.numel() < (n - 1) * source_stride + rows:
+            if source_stride < 0 or source.numel() < (n - 1) * source_stride + rows or \
+                    source.dtype != _torch().float64 or not source.is_contiguous() or \
+                    source.device != d.device:
                 raise ValueError("source: contiguous FP64 on the device, stage s's %d values "
                                  "from s * source_stride" % rows)
             cptr, sptr = self._field_ptrs(coeff, None)[0], source.data_ptr()
@@ -772,33 +774,40 @@ class CompiledOperator:
         with the state q [F, K*Np] of any real type (hb_adjoint_stage: two
         launches; where that refuses, beyond order 7, composed from
         ``adjoint``)."""
+        self.adjoint_step((a,), (b,), dt, lam, lq, (q,), coeff, c_bar)
+
+    def adjoint_step(self, a, b, dt, lam, lq, states, coeff=None, c_bar=None):
+        """The stages of a step reversed, the last first: ``adjoint_stage``
+        with a[s], b[s] at the state states[s]."""
         d = self.discr
-        n, f64 = len(d), _torch().float64
-        c = self._coeff if coeff is None else coeff
-        for name, x, size in (("lam", lam, self.F * n), ("lq", lq, self.F * n),
-                              ("c_bar", c_bar, n), ("coeff", coeff, n)):
+        n, f64, device = len(d), _torch().float64, d.device
+        size = self.F * n
+        for name, x, m in (("lam", lam, size), ("lq", lq, size), ("c_bar", c_bar, n),
+                           ("coeff", coeff, n)):
             if x is not None and (x.dtype != f64 or not x.is_contiguous() or
-                                  x.numel() != size or x.device != d.device):
-                raise ValueError("%s: contiguous FP64 [%d] on the device" % (name, size))
-        if q is not None and (q.dtype != f64 or not q.is_contiguous() or
-                              q.numel() != self.F * n or q.device != d.device):
-            q = q.to(device=d.device, dtype=f64).reshape(self.F, n).contiguous()
-        st = self._lib.hb_adjoint_stage(
-            self._handle, float(a), float(b), float(dt),
-            q.data_ptr() if q is not None else None, lam.data_ptr(), lq.data_ptr(),
-            c_bar.data_ptr() if c_bar is not None else None,
-            c.data_ptr() if c is not None else None, self._adjoint_work().data_ptr(),
-            self._stream())
-        if st != _native.HB_ERR_UNSUPPORTED:
-            _native.check(st)
-            return
-        lam, lq = lam.view(self.F, n), lq.view(self.F, n)
-        lam.add_(lq, alpha=b)
-        q_bar, cb = self.adjoint(lam, q=q, coeff=coeff, want_c=c_bar is not None)
-        lq.add_(q_bar, alpha=dt)
-        if c_bar is not None:
-            c_bar.view(n).add_(cb, alpha=dt)
-        lam.mul_(a)
+                                  x.numel() != m or x.device != device):
+                raise ValueError("%s: contiguous FP64 [%d] on the device" % (name, m))
+        c = self._coeff if coeff is None else coeff
+        call, work, stream = self._lib.hb_adjoint_stage, self._adjoint_work(), self._stream()
+        ptrs = (lam.data_ptr(), lq.data_ptr(), c_bar.data_ptr() if c_bar is not None else None,
+                c.data_ptr() if c is not None else None, work.data_ptr(), stream)
+        for s in range(len(states) - 1, -1, -1):
+            q = states[s]
+            if q is not None and (q.dtype != f64 or not q.is_contiguous() or
+                                  q.numel() != size or q.device != device):
+                q = q.to(device=device, dtype=f64).reshape(self.F, n).contiguous()
+            st = call(self._handle, float(a[s]), float(b[s]), float(dt),
+                      q.data_ptr() if q is not None else None, *ptrs)
+            if st == _native.HB_ERR_UNSUPPORTED:
+                lam, lq = lam.view(self.F, n), lq.view(self.F, n)
+                lam.add_(lq, alpha=b[s])
+                q_bar, cb = self.adjoint(lam, q=q, coeff=coeff, want_c=c_bar is not None)
+                lq.add_(q_bar, alpha=dt)
+                if c_bar is not None:
+                    c_bar.view(n).add_(cb, alpha=dt)
+                lam.mul_(a[s])
+            else:
+                _native.check(st)
 
     def check(self):
         """Synchronise and raise if a kernel flagged bad input."""
@@ -916,16 +925,21 @@ class BoundRHS:
         no boundary data or velocity to evaluate, or this class and the model
         evaluate it in their own ``context`` (not an override) and all that
         it reads are TimeConstantGivenFunctions."""
-        if getattr(self.context, "__func__", None) is not BoundRHS.context:
+        if type(self).context is not BoundRHS.context or "context" in self.__dict__:
             return False
         comp = self.compiled
         if not comp.n_given and comp.ot.model != MODEL_VARADV:
             return True
         ctx = getattr(self.model, "context", None)
         read = CONTEXT_DATA.get(getattr(ctx, "__func__", None))
-        return read is not None and all(
-            x is None or isinstance(x, str) or type(x) is TimeConstantGivenFunction
-            for x in (getattr(ctx.__self__, name) for name in read))
+        if read is None:
+            return False
+        for name in read:
+            x = getattr(ctx.__self__, name)
+            if type(x) is not TimeConstantGivenFunction and x is not None and \
+                    not isinstance(x, str):
+                return False
+        return True
 
     def __call__(self, t, w, **extra_context):
         kw = self.context(t)

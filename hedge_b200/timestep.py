@@ -39,10 +39,9 @@ _TABLE_BYTES = _TABLE.tobytes()
 
 def _stage_arrays(coeffs):
     """The a and b columns of a coefficient table for the native step."""
-    table = np.asarray(coeffs, dtype=np.float64)
-    if table.tobytes() == _TABLE_BYTES:
+    if type(coeffs) is np.ndarray and coeffs.tobytes() == _TABLE_BYTES:
         return _A, _B
-    a, b, _ = table.T.tolist()
+    a, b, _ = np.asarray(coeffs, dtype=np.float64).T.tolist()
     return (C.c_double * len(a))(*a), (C.c_double * len(b))(*b)
 
 
@@ -69,7 +68,7 @@ class LSRK4TimeStepper:
             if rhs.constant_context():
                 # the model's data evaluated once, the stages in one call
                 a, b = _stage_arrays(self.coeffs)
-                stages = [y] + [bufs[s % 2] for s in range(len(a))]
+                stages = [y] + (bufs * len(a))[:len(a)]
                 comp.lsrk_step(a, b, dt, stages, self.residual, **rhs.context(t))
                 return stages[-1]
             cur = y

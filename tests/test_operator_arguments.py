@@ -91,6 +91,13 @@ def test_adjoint_stage_takes_device_vectors():
     assert name == "hb_adjoint_stage" and args[4] not in (None, q.data_ptr())
 
 
+def test_adjoint_step_takes_the_stages_last_first():
+    op = _operator()
+    op.adjoint_step((0.1, 0.2), (0.3, 0.4), 0.5, _vec(F, N), _vec(F, N), (_vec(F, N), None))
+    assert [(c[1][1], c[1][2]) for c in op._lib.calls] == [(0.2, 0.4), (0.1, 0.3)]
+    assert op._lib.calls[0][1][4] is None and op._lib.calls[1][1][4] is not None
+
+
 @pytest.mark.parametrize("bad", [_vec(F, N, dtype=torch.float32), _vec(F, N - 1), _vec(N, F).T,
                                  _vec(F, 2 * N)[:, ::2], torch.ones(1, 1).double().expand(F, N)])
 @pytest.mark.parametrize("which", ["lam", "lq"])

@@ -29,12 +29,13 @@ class _Linear:
             res.mul_(a[s]).sub_(bufs[s], alpha=dt)
             bufs[s + 1].copy_(bufs[s]).add_(res, alpha=b[s])
 
-    def adjoint_stage(self, a, b, dt, lam, lq, q=None, coeff=None, c_bar=None):
+    def adjoint_step(self, a, b, dt, lam, lq, states, coeff=None, c_bar=None):
         for x in (lam, lq):
             assert x.dtype == torch.float64 and x.is_contiguous() and x.shape == (F, N)
-        lam.add_(lq, alpha=b)
-        lq.sub_(lam, alpha=dt)
-        lam.mul_(a)
+        for s in reversed(range(len(states))):
+            lam.add_(lq, alpha=b[s])
+            lq.sub_(lam, alpha=dt)
+            lam.mul_(a[s])
 
 
 class _Plain:
