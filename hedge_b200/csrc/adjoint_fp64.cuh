@@ -25,11 +25,11 @@
 // forms lam in place, the element kernel reads only its own element's and
 // writes the rest, so that a stage is two launches and no vector passes.
 //
-// Bound: launch latency and the point phases.  Measured against one block per
-// element with the operators read by thread rows: variable-velocity wave with
-// the c gradient, 2D, K = 7200, N = 5, 61 us for both passes before; 8 LSRK4
-// steps with receivers forward and backward at K = 2112, N = 4, 5.2 -> 3.0 ms
-// (of which the vector passes of the recurrences took half).
+// Bound: launch latency and the point phases.  Both passes, against one block
+// per element with the operators read by thread rows: variable-velocity wave
+// with the c gradient, 2D, K = 7200, N = 5, 55 -> 20 us, K = 24200 156 -> 79 us; 3D, K =
+// 1296, N = 4 77 -> 20 us; 3D Maxwell, K = 6000, N = 4 283 -> 81 us.  8 LSRK4 steps with
+// receivers forward and backward at K = 2112, N = 4 take half of the time before.
 #pragma once
 
 #include <algorithm>

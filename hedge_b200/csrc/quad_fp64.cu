@@ -16,7 +16,7 @@
 //
 // Bound: FP64 pipe (N = 5, 64 volume points: 294 MMAs per 8 elements, 40 us at
 // K = 80000) and L1 wavefronts of the scattered 8-byte gathers.  A stage at K =
-// 80000, N = 5: 219 -> 72 us, N = 3 66 -> 36, N = 7 1178 -> 249 (rhs_quad.cu -> here); the
+// 80000, N = 5: 222 -> 69 us, N = 3 65 -> 37, N = 7 1185 -> 247 (rhs_quad.cu -> here); the
 // sizes and meshes that stay there are in quad_on_cores.  The element sizes are
 // run-time values except the number of 8-node tiles KS.
 #include <algorithm>
@@ -333,7 +333,7 @@ hb_status prepare_quad_f64(Op* op, const hb_quad_desc* qd) {
   // the points that pad a tile repeat the last one, against zeros in the
   // projection and the lift: as 0 * w their values would not be zero where w is
   // not finite, also where the flux of the points does not see that w
-  // (selecting zeros in the kernel instead: 72 -> 76 us a stage at N = 5, K = 80000)
+  // (selecting zeros in the kernel instead: 69 -> 72 us a stage at N = 5, K = 80000)
   for (int q = 0; q < 8 * nqt; ++q)
     for (int j = 0; j < np; ++j)
       I[at((size_t)(q / 8) * ks + j / 8, q % 8, j % 8)] =

@@ -16,7 +16,8 @@
 // integrals, and the face integrals carry Fscale = face Jacobian / |J|.
 //
 // This file's kernel runs on the CUDA cores, for the element sizes that the
-// FP64 tensor-core form (quad_fp64.cu) is not built for.  One persistent CTA
+// FP64 tensor-core form (quad_fp64.cu) is not built for and the meshes that are
+// faster here (quad_on_cores).  One persistent CTA
 // of 256 threads loops over batches of E elements:
 //   A. stage u and v (all components) of the batch in shared memory
 //      (coalesced), the geometry and the face table;

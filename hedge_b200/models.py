@@ -424,7 +424,7 @@ class MaxwellOperator(HyperbolicOperator):
         (every kernel); incident data given per call as boundary vectors
         (template fields outside any BoundarizeOperator, one per carried
         component, e.g. ``make_sym_vector("inc", n_fields)``) runs on the
-        fp64 and fp32 CUDA-core kernels."""
+        kernels of fp64 and of fp32 on the CUDA cores."""
         self.dimensions = dimensions or self._default_dimensions
         if self.dimensions != self._default_dimensions:
             raise NotImplementedError("%s is a %dD system" % (type(self).__name__,

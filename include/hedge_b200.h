@@ -51,7 +51,8 @@ enum {
 enum {
   HB_PREC_FP64 = 0,   /* FP64 state, FP64 arithmetic */
   HB_PREC_FP32 = 1,   /* FP32 state and residual.  In 2D and up to order 3 in 3D the
-                         arithmetic is FP64 (FP64 tensor cores); where a resident
+                         arithmetic is FP64 (FP64 tensor cores; CUDA cores for
+                         advection of low order on larger meshes); where a resident
                          tensor-core kernel is built for the (model, dimension, order)
                          beyond that (and, on large meshes, for the sizes it is faster
                          at) the two contractions are FP16-split products of scaled rows
